@@ -72,9 +72,8 @@
  *  PF_BINS_SHARED  (CE / AOV, chosen) keep the shared-histogram binning
  *                  (one histogram per warp and trial period, filled with
  *                  shared atomics) for the length classes it serves (curves
- *                  shorter than 1024 points) instead of letting the
- *                  autotuner weigh it against per-thread privatised
- *                  histograms.  Values are identical either way.
+ *                  shorter than 1024 points) instead of the per-thread
+ *                  privatised histograms.  Values are identical either way.
  *  PF_ONE_LAUNCH   (chosen) run every curve in one launch with the shape
  *                  tuned for the length class holding the most points,
  *                  instead of one launch per class with its own tuned shape

@@ -217,6 +217,7 @@ struct pf_ctx {
         int block;
         bool persist;
         int rounds;
+        int cells;
         float ms;        // sample time of the winner
         float ms_worst;  // and of the slowest candidate
         uint32_t candidates;
@@ -613,6 +614,7 @@ FoldConfig choose_config(pf_ctx* ctx, const Job& j, uint32_t max_len, bool& ok) 
     c.acc = AOVACC_F32;
     c.n_sm = ctx->n_sm;
     c.rounds = 1;
+    c.cells = 1;
     c.ovl = (j.algo == ALGO_CE) ? (j.po > 1 || j.mo > 1) : (j.algo == ALGO_AOV && j.po > 1);
     if (chosen && !c.ovl && (j.algo == ALGO_CE || j.algo == ALGO_AOV) && max_len < 65536u) {
         c.kind = KIND_BIN;
@@ -625,6 +627,20 @@ FoldConfig choose_config(pf_ctx* ctx, const Job& j, uint32_t max_len, bool& ok) 
         c.acc = AOVACC_FIX;
     }
     ok = false;
+    if (c.kind == KIND_BIN && !c.ref_stats) {
+        // Without tuning: two periods per thread in small CTAs (the shape
+        // tuning mostly picks), fewer where the histograms are large.
+        const int shapes[4][2] = {{64, 2}, {32, 2}, {64, 1}, {32, 1}};
+        for (const auto& sh : shapes) {
+            c.block = sh[0];
+            c.cells = sh[1];
+            if (fold_smem(c, j.n_phase, j.n_mag) <= ctx->smem_optin) {
+                ok = true;
+                return c;
+            }
+        }
+        return c;
+    }
     int best_warps = 0;
     const int blocks[3] = {256, 128, 64};
     for (int b : blocks) {
@@ -739,7 +755,8 @@ int plan(pf_ctx* ctx, const Job& j, const uint64_t* lengths, bool with_points, b
         return fail(ctx, PF_EUNSUPPORTED,
                     "histogram of %u x %u bins does not fit in shared memory", j.n_phase,
                     j.algo == ALGO_CE ? j.n_mag : 1u);
-    const uint64_t tiles_per = (j.n_per + cfg.block - 1) / cfg.block;
+    const uint64_t per_item = (uint64_t)item_periods(cfg);
+    const uint64_t tiles_per = (j.n_per + per_item - 1) / per_item;
     const uint64_t n_work64 = j.n_curves * j.n_pdt * tiles_per;
     if (n_work64 > 0x7FFFFFFFull) return fail(ctx, PF_EINVAL, "too much work for one launch");
     L.n_work = (uint32_t)n_work64;
@@ -854,8 +871,10 @@ cudaError_t launch_fold_sem(const Job& j, const FoldConfig& c, const FoldParams&
 }
 
 // Launch shape of one length class.  Cached per context; the first time a
-// key is met, every candidate (block 64 / 128 / 256 where shared memory
-// allows, persistent or one CTA per item) is timed with CUDA events on a
+// key is met, every candidate (the bin kernel: block 32 / 64 / 128 where
+// shared memory allows, 1 or 2 periods per thread at once, in 1 or 4 rounds;
+// the others: block 64 / 128 / 256, persistent or one CTA per item) is timed
+// with CUDA events on a
 // sample of the class (a contiguous run of its curves from the middle of
 // the class, about 2e9 point evaluations) and the fastest kept.  The sample
 // writes cells of the real output, which the class launch rewrites.  Every
@@ -871,11 +890,12 @@ int tuned_config(pf_ctx* ctx, const Job& j, const FoldConfig& base, int cls, uin
     const bool rec_ok = j.fgrid && base.algo == ALGO_LS && base.fold == FOLD_DF;
     const bool only_rec = rec_ok && (j.mode & PF_TRIG_RECURRENCE);
     const bool no_rec = !rec_ok || (j.mode & PF_TRIG_SINCOS);
-    // Likewise the binning strategy of the chosen CE / AOV kernels:
-    // per-thread privatised histograms, or shared histograms with atomics
-    // (PF_BINS_SHARED keeps the latter where the curves fit it).
-    const bool warp_ok = base.kind == KIND_BIN && !base.ref_stats && cls <= kWarpClassMax;
-    const bool only_warp = warp_ok && (j.mode & PF_BINS_SHARED);
+    // PF_BINS_SHARED takes the shared-histogram binning where the curves fit
+    // it.  It is no candidate otherwise: its samples were 1.3-5x the
+    // privatised form's on every class measured, before that form's newer
+    // shapes.
+    const bool only_warp = base.kind == KIND_BIN && !base.ref_stats && cls <= kWarpClassMax &&
+                           (j.mode & PF_BINS_SHARED);
     if (only_rec) {
         out.kind = KIND_LSREC;
         out.block = 256;
@@ -895,6 +915,7 @@ int tuned_config(pf_ctx* ctx, const Job& j, const FoldConfig& base, int cls, uin
         out.block = it->second.block;
         out.persist = it->second.persist;
         out.rounds = it->second.rounds;
+        out.cells = it->second.cells;
         return PF_OK;
     }
     if (j.mode & PF_NO_TUNE) return PF_OK;
@@ -917,28 +938,32 @@ int tuned_config(pf_ctx* ctx, const Job& j, const FoldConfig& base, int cls, uin
     ps.bins = nullptr;
     ps.q.order = p.q.order + s0;
     ps.q.next = reinterpret_cast<unsigned*>((char*)ctx->d_misc.p + kCounterOffset) + kTuneCounter;
-    pf_ctx::Tuned best{out.kind, out.block, out.persist, out.rounds, 1e30f, 0.0f, 0};
-    // Candidates: block x persistent-or-not, and for the bin kernel 1 or 4
-    // rounds of periods per item; for the recurrence 4 or 8 frequencies per
+    pf_ctx::Tuned best{out.kind, out.block, out.persist, out.rounds, out.cells, 1e30f, 0.0f, 0};
+    // Candidates: see above; for the recurrence 4 or 8 frequencies per
     // thread.  The reference statistic is built in one shape only.
     std::vector<FoldConfig> cands;
     const bool shapes = !(base.kind == KIND_BIN && base.ref_stats);
     if (!only_rec && !only_warp) {
-        for (int block : {64, 128, 256}) {
+        const bool bin = base.kind == KIND_BIN && shapes;
+        for (int block : {32, 64, 128, 256}) {
+            if (block == (bin ? 256 : 32)) continue;
             FoldConfig t = base;
             t.block = block;
-            if (fold_smem(t, j.n_phase, j.n_mag) > ctx->smem_optin) continue;
-            for (int shape = 0; shape < (shapes ? 4 : 1); shape++) {
-                t.persist = (shape & 1) != 0;
-                t.rounds = (base.kind == KIND_BIN && (shape & 2)) ? 4 : 1;
-                if (base.kind != KIND_BIN && (shape & 2)) continue;
-                cands.push_back(t);
+            for (int cells : {1, 2}) {
+                if (!bin && cells > 1) continue;
+                t.cells = cells;
+                if (fold_smem(t, j.n_phase, j.n_mag) > ctx->smem_optin) continue;
+                // bin kernel: 1 or 4 rounds; others: persistent or not
+                for (int alt = 0; alt < (shapes ? 2 : 1); alt++) {
+                    t.rounds = bin && alt ? 4 : 1;
+                    t.persist = !bin && alt;
+                    cands.push_back(t);
+                }
             }
         }
     }
-    // The shared-histogram binning (one histogram per warp and period,
-    // shared atomics) for classes of curves shorter than its staging limit.
-    if (warp_ok) {
+    // The shared-histogram binning (one histogram per warp and period).
+    if (only_warp) {
         for (int block : {128, 256})
             for (int persist = 0; persist < 2; persist++) {
                 FoldConfig t = base;
@@ -1014,6 +1039,7 @@ int tuned_config(pf_ctx* ctx, const Job& j, const FoldConfig& base, int cls, uin
             best.block = c.first.block;
             best.persist = c.first.persist;
             best.rounds = c.first.rounds;
+            best.cells = c.first.cells;
         }
     }
     ctx->tuned[key] = best;
@@ -1021,6 +1047,7 @@ int tuned_config(pf_ctx* ctx, const Job& j, const FoldConfig& base, int cls, uin
     out.block = best.block;
     out.persist = best.persist;
     out.rounds = best.rounds;
+    out.cells = best.cells;
     return PF_OK;
 }
 
@@ -1119,6 +1146,9 @@ int device_pipeline(pf_ctx* ctx, const Job& j, const Layout& L, const FoldConfig
     p.mag_bin_size = bin_size(j.n_mag, cpu);
     p.out = d_out;
     p.edge_d = edge_guard(j.n_phase);
+    const uint32_t edge32 = (p.edge_d << 12) / j.n_phase + 2u;  // D
+    p.magic32 = 6755399441055744.0 + (double)edge32;
+    p.edge32_lim = 2u * edge32 * j.n_phase;
     p.fgrid = j.fgrid ? 1 : 0;
     p.f0 = j.f0;
     p.df = j.df;
@@ -1136,15 +1166,48 @@ int device_pipeline(pf_ctx* ctx, const Job& j, const Layout& L, const FoldConfig
         ctx->launches++;
     }
     if (cfg.kind == KIND_BIN && j.algo == ALGO_CE) {
-        if ((rc = ensure_dev(ctx, ctx->d_aux64, L.total_pts * 8 + 32)) != PF_OK) return rc;
-        p.aux64 = (const uint64_t*)ctx->d_aux64.p;
-        cudaError_t e = cpu ? launch_binaux_cpusem(p.m, ctx->d_aux64.p, dcurves, ncur, j.n_mag,
-                                                   p.mag_bin_size, cfg.block, cfg.cnt16, s)
-                            : launch_binaux_cudasem(p.m, ctx->d_aux64.p, dcurves, ncur,
-                                                    j.n_mag, p.mag_bin_size, cfg.block,
-                                                    cfg.cnt16, s);
-        PF_CUDA(e, "CE bin preparation kernel");
+        // Sorted times and run tables: a fixed stride per curve where that
+        // is small (few magnitude columns against the curve lengths), else
+        // by the curve's own length, which bounds its runs.
+        CeSortLayout lay{1, (3 * j.n_mag + 3) & ~3u, 0, j.n_mag + 2};
+        size_t n_ts = L.total_pts + (size_t)ncur * lay.ts_pad;
+        size_t n_runs = (size_t)ncur * lay.run_pad;
+        if (n_ts > 4 * L.total_pts + (1u << 20)) {
+            lay.ts_mul = 4;
+            lay.ts_pad = 0;
+            n_ts = 4 * L.total_pts;
+        }
+        if (n_runs > L.total_pts + 4 * (size_t)ncur + (1u << 20)) {
+            lay.run_mul = 1;
+            lay.run_pad = 4;
+            n_runs = L.total_pts + 4 * (size_t)ncur;
+        }
+        const size_t o_runs = align_up(n_ts * 4 + 32, 256);
+        if ((rc = ensure_dev(ctx, ctx->d_aux32, o_runs + n_runs * 4)) != PF_OK) return rc;
+        float* ts = (float*)ctx->d_aux32.p;
+        uint32_t* runs = (uint32_t*)((char*)ctx->d_aux32.p + o_runs);
+        p.ts = ts;
+        p.runs = runs;
+        p.ts_mul = lay.ts_mul;
+        p.ts_pad = lay.ts_pad;
+        p.run_mul = lay.run_mul;
+        p.run_pad = lay.run_pad;
+        PF_CUDA(cpu ? launch_cesort_cpusem(p.t, p.m, dcurves, ncur, j.n_mag, p.mag_bin_size, lay,
+                                           ts, runs, s)
+                    : launch_cesort_cudasem(p.t, p.m, dcurves, ncur, j.n_mag, p.mag_bin_size,
+                                            lay, ts, runs, s),
+                "CE sort kernel");
         ctx->launches++;
+        if (j.mode & PF_BINS_SHARED) {
+            if ((rc = ensure_dev(ctx, ctx->d_aux64, L.total_pts * 8 + 32)) != PF_OK) return rc;
+            p.aux64 = (const uint64_t*)ctx->d_aux64.p;
+            PF_CUDA(cpu ? launch_binaux_cpusem(p.m, ctx->d_aux64.p, dcurves, ncur, j.n_mag,
+                                               p.mag_bin_size, s)
+                        : launch_binaux_cudasem(p.m, ctx->d_aux64.p, dcurves, ncur, j.n_mag,
+                                                p.mag_bin_size, s),
+                    "CE bin preparation kernel");
+            ctx->launches++;
+        }
     } else if (cfg.kind == KIND_BIN && j.algo == ALGO_AOV) {
         if ((rc = ensure_dev(ctx, ctx->d_aux32, L.total_pts * 4 + 16)) != PF_OK) return rc;
         p.aux32 = (const uint32_t*)ctx->d_aux32.p;
@@ -1755,7 +1818,8 @@ size_t pfk::fold_smem(const FoldConfig& c, uint32_t n_phase, uint32_t n_mag) {
     if (c.kind == KIND_BINWARP)
         return (size_t)kWarpMaxPoints * 16 +
                (size_t)(c.block / 32) * (c.algo == ALGO_CE ? n_phase * n_mag : 2 * n_phase) * 4;
-    if (c.kind == KIND_BIN) return bin_smem_bytes(c.algo, c.cnt16, c.block, n_phase, n_mag);
+    if (c.kind == KIND_BIN)
+        return bin_smem_bytes(c.algo, c.cnt16, c.block * std::max(c.cells, 1), n_phase, n_mag);
     return fold_smem_bytes(c.algo, c.fold, c.acc, c.block, c.ovl, n_phase, n_mag);
 }
 
@@ -1893,7 +1957,7 @@ int pf_tuning_report(const pf_ctx* ctx, char* buf, uint64_t len) {
     for (const auto& kv : ctx->tuned) {
         char line[320];
         snprintf(line, sizeof(line),
-                 "%s: %sblock=%d rounds=%d %s sample_ms=%.3f slowest_ms=%.3f candidates=%u\n",
+                 "%s: %sblock=%d rounds=%d cells=%d %s sample_ms=%.3f slowest_ms=%.3f candidates=%u\n",
                  kv.first.c_str(),
                  kv.second.kind == KIND_LSREC ? "trig=recurrence "
                  : kv.second.kind == KIND_BINWARP ? "bins=shared-atomic "
@@ -1901,7 +1965,7 @@ int pf_tuning_report(const pf_ctx* ctx, char* buf, uint64_t len) {
                  : (kv.second.kind == KIND_FOLD && kv.first.find("fgrid") != std::string::npos)
                      ? "trig=sincos "
                      : "",
-                 kv.second.block, kv.second.rounds,
+                 kv.second.block, kv.second.rounds, std::max(kv.second.cells, 1),
                  kv.second.persist ? "persistent" : "one-cta-per-item", kv.second.ms,
                  kv.second.ms_worst, kv.second.candidates);
         out += line;

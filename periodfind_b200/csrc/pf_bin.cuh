@@ -25,19 +25,46 @@
 // Valid while |q| * n < 2^30 (checked per CTA from the batch's max|t|;
 // otherwise the CTA runs the generic loop).  While also |q| < 2^19 one FP64
 // operation does it (fast_bin32): y = RD(t_corr * (RN(1/P) * 2^32) +
-// 1.5*2^52) on the exact product leaves floor(frac(q') * 2^32) in its low
-// word f, and the 64-bit product f * n holds the row (high word) and the
-// position within it (low word, tested against the same guard in units of
-// 2^-32, widened by n + 2 for the truncation).
+// 1.5*2^52 + D) on the exact product leaves floor(frac(q') * 2^32) + D in its
+// low word f, and the 64-bit product f * n holds the row (high word) and the
+// position within it (low word, the edge test: D puts the guard below it).
 //
-// CE counters are 16-bit halves of 32-bit words when every count fits
-// (curve length * overlaps < 65536), doubling the CTAs per SM; AOV keeps a
+// CE counters are 16-bit halves of 32-bit words (curve length * overlaps <
+// 65536), doubling the cells per SM; AOV keeps a
 // 32-bit count and a 32-bit fixed-point magnitude sum per bin.  Updates are
 // `red.shared.add.u32` (no return value, no dependency chain).
+//
+// What bounds it: the shared-memory pipe.  Every lane of a warp reads the
+// same staged point, and a 128-bit broadcast load occupies the pipe about
+// 2.6 times as long as a conflict-free reduction (1.62 against 0.62 in the
+// same units, 32 warps per SM), so one 16-byte point record and one
+// reduction per evaluation were bound by the load.  Three things shrink it:
+//   - CE takes its points sorted by magnitude column (ce_sort_kernel), so a
+//     point is its time alone and the counter word and increment stay in
+//     registers for a column's run;
+//   - a thread holds CELLS = 2 periods, so one load serves two evaluations
+//     (4 were slower: 96-128 registers at 10 warps per SM);
+//   - the guard rides in the FMA's constant and the product is one wide
+//     multiply, so an evaluation is DFMA, IMAD.WIDE, IMAD, RED and half a
+//     three-way minimum (6.4 instructions with all overheads on 4096 points,
+//     11.1 before).
+// Measured, 3000 ragged curves (20-2000 points) x 20000 periods, CE 10 x 10
+// then AOV 15, plan with peaks: 12.06 -> 10.50 ms and 11.63 -> 9.05 ms;
+// CE 200 x 4096 x 10000 x 2 derivatives 7.26 -> 5.27 ms.  CE [1024,4096):
+// issue 61%, fmaheavy pipe 73%, shared-memory pipe 50%; AOV: shared-memory
+// pipe 88% (its two reductions per evaluation).
 #pragma once
 
 namespace pfk {
 namespace PF_KNS {
+
+// Resident CTAs per SM the bin kernel is compiled for: 1024 cells (CE, the
+// shared-memory limit of 10 x 10 counters) and 1280 (AOV; 1024 measured 2-3%
+// slower) per SM.
+template <int ALGO, int BLOCK, int CELLS>
+constexpr int bin_min_blocks() {
+    return (ALGO == ALGO_CE ? 1024 : 1280) / (BLOCK * CELLS);
+}
 
 // Fire-and-forget shared reduction.  No "memory" clobber: the counters it
 // updates are never read inside the point loop, so the compiler may hoist
@@ -46,6 +73,15 @@ namespace PF_KNS {
 // compiler barrier plus __syncwarp().
 __device__ __forceinline__ void red_shared_u32(uint32_t addr, uint32_t v) {
     asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(addr), "r"(v));
+}
+
+// Both halves of a 32 x 32 bit product from one wide multiply (written as a
+// C++ 64-bit product the compiler took a low and a high multiply).
+__device__ __forceinline__ void mul_wide_u32(uint32_t a, uint32_t b, uint32_t& lo,
+                                             uint32_t& hi) {
+    asm("{ .reg .u64 w; mul.wide.u32 w, %2, %3; mov.b64 {%0, %1}, w; }"
+        : "=r"(lo), "=r"(hi)
+        : "r"(a), "r"(b));
 }
 
 __device__ __forceinline__ void compiler_fence() { asm volatile("" ::: "memory"); }
@@ -58,11 +94,8 @@ __device__ __forceinline__ uint32_t lds_u32(uint32_t addr) {
 
 constexpr double kMagic15 = 6755399441055744.0;  // 1.5 * 2^52
 
-// One CTA: curve w.curve, period derivative w.pdt, periods p0 .. p0+np-1
-// (one per thread).  Shared memory: [tile of 16-byte point records
-// {double t; u32 a; u32 b}][counters].  CE: a = byte offset of the
-// magnitude column within a phase row, b = increment (1 or 1 << 16).
-// AOV: a = fixed-point magnitude.
+// A staged point of the shared-histogram kernel (pf_binwarp.cuh): its time,
+// and its magnitude bin (CE) or fixed-point magnitude (AOV).
 struct BinPoint {
     double t;
     uint32_t a, b;
@@ -112,7 +145,7 @@ __device__ __forceinline__ float ce_stat_fast(uint32_t tbase, uint32_t nP, uint3
         uint32_t col = 0;
         float row = 0.0f;
         for (uint32_t wi = 0; wi < W; wi++) {
-            const uint32_t wv = lds_u32(tbase + (j * W + wi) * block * 4u);
+            const uint32_t wv = lds_u32(tbase + (wi * nP + j) * block * 4u);
             if constexpr (CNT16) {
                 // Both 16-bit halves summed at once: each half's column
                 // total is at most n < 2^16, so no carry crosses halves.
@@ -152,16 +185,15 @@ __device__ __forceinline__ double aov_sbx_fast(uint32_t tbase, uint32_t nP, uint
 //         summed, with the 1/n scale taken out of the logs);
 //   AOV = (n - nP)/(nP - 1) * s1 / s2, s1 = sum_b X_b^2 / c_b - X^2 / n,
 //         s2 = sum x^2 - sum_b X_b^2 / c_b (X_b the fixed-point bin sums).
-template <int ALGO, bool CNT16, int BLOCK, bool REF_STATS, int ROUNDS>
+template <int ALGO, bool CNT16, int BLOCK, bool REF_STATS, int ROUNDS, int CELLS>
 __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, uint32_t item) {
     extern __shared__ __align__(16) unsigned char smem[];
-    // CE: one 16-byte record per point.  AOV: the times (doubles) and the
-    // fixed-point magnitudes in two arrays, so four points take three
-    // 128-bit loads instead of four.
-    BinPoint* tile = reinterpret_cast<BinPoint*>(smem);
+    constexpr uint32_t kCols = BLOCK * CELLS;  // counter columns of the CTA
+    // CE: the times of the staged points (doubles), sorted by magnitude
+    // column.  AOV: the times and the fixed-point magnitudes.
     double* tile_t = reinterpret_cast<double*>(smem);
     uint32_t* tile_a = reinterpret_cast<uint32_t*>(smem + kBinTile * sizeof(double));
-    unsigned char* cnt_raw = smem + kBinTile * sizeof(BinPoint);
+    unsigned char* cnt_raw = smem + bin_tile_bytes(ALGO);
     const uint32_t cnt_base = (uint32_t)__cvta_generic_to_shared(cnt_raw);
 
     stamp_start(p, item);
@@ -171,17 +203,18 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
     const float period_dt = p.pdts[w.pdt];
     const uint32_t nP = p.n_phase, nM = p.n_mag;
 
-    // Counter layout: CE  [nP rows][W words][BLOCK] u32, W = nM or ceil(nM/2)
-    //                 AOV [nP][2][BLOCK] u32 (count, fixed-point sum): a bin's
-    //                 sum lies a constant BLOCK words after its count, so the
+    // Counter layout: CE  [W words][nP rows][kCols] u32, W = nM or ceil(nM/2)
+    //                 AOV [nP][2][kCols] u32 (count, fixed-point sum): a bin's
+    //                 sum lies a constant kCols words after its count, so the
     //                 second reduction takes an immediate address offset.
+    // Cell c of thread tid owns column c * BLOCK + tid.
     const uint32_t W = (ALGO == ALGO_CE) ? (CNT16 ? (nM + 1) / 2 : nM) : 1;
-    const uint32_t row_stride = W * BLOCK * 4;  // bytes per phase row
     const uint32_t slots = (ALGO == ALGO_CE) ? nP * W : 2 * nP;
     const uint32_t tbase = cnt_base + tid * 4;
 
-    // The item covers ROUNDS x BLOCK periods; thread tid takes period
-    // p0 + r * BLOCK + tid in round r.  Range guard for y = q * n * 2^20 over
+    // The item covers ROUNDS x CELLS x BLOCK periods; in round r thread tid
+    // takes periods p0 + (r * CELLS + c) * BLOCK + tid, c < CELLS, all at
+    // once.  Range guard for y = q * n * 2^20 over
     // every round (uniform over the CTA).  The cell constants (1 / P as a
     // double-double, pdt / 2P) are finite exactly when P is finite and non-zero
     // and pdt is finite; non-finite periods or derivatives (device-pointer
@@ -190,7 +223,7 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
     bool fin = isfinite(period_dt);
     double my_pmin = INFINITY;
 #pragma unroll
-    for (int r = 0; r < ROUNDS; r++) {
+    for (int r = 0; r < ROUNDS * CELLS; r++) {
         const uint32_t j = (uint32_t)(r * BLOCK + tid);
         const float per = p.periods[w.p0 + (j < w.np ? j : 0u)];
         fin = fin && isfinite(per) && per != 0.0f;
@@ -207,59 +240,76 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
     // the fraction bits moved to the top of the word.
     const uint32_t edge_add = p.edge_d << 12;
     const uint32_t edge_lim = (2u * p.edge_d) << 12;
-    // The same guard in units of 2^-32 of a bin for fast_bin32, widened by
-    // n_phase + 2 units for the truncation of the phase to 32 bits.
-    const uint32_t edge32_add = edge_add + nP + 2u;
-    const uint32_t edge32_lim = 2u * edge32_add;
+    const uint32_t edge32_lim = p.edge32_lim;
+
+    // CE: the curve's sorted times and its runs of equal magnitude column
+    // (see ce_sort_kernel).  n_pad counts the runs' padding.
+    const float* src_t = p.t + cd.off;
+    const uint32_t* runs = nullptr;
+    uint32_t n_pad = n;
+    if constexpr (ALGO == ALGO_CE) {
+        src_t = p.ts + (cd.off * p.ts_mul + (int64_t)w.curve * p.ts_pad);
+        runs = p.runs + (cd.off * p.run_mul + (int64_t)w.curve * p.run_pad);
+        n_pad = runs[0];
+    }
 
     auto stage = [&](uint32_t base, uint32_t cnt) {
-        const float4* gt = reinterpret_cast<const float4*>(p.t + cd.off + base);
+        const float4* gt = reinterpret_cast<const float4*>(src_t + base);
         const uint32_t n4 = (cnt + 3) >> 2;
-        if constexpr (ALGO == ALGO_CE) {
-            const uint4* ga = reinterpret_cast<const uint4*>(p.aux64 + cd.off + base);
-            for (uint32_t i4 = tid; i4 < n4; i4 += BLOCK) {
-                const float4 q = gt[i4];
-                const uint4 a01 = ga[2 * i4], a23 = ga[2 * i4 + 1];
-                // Counter word within a phase row -> byte offset for this
-                // CTA shape (the prepared data does not depend on BLOCK).
-                constexpr uint32_t kColBytes = BLOCK * 4u;
-                tile[4 * i4 + 0] = BinPoint{(double)q.x, a01.x * kColBytes, a01.y};
-                tile[4 * i4 + 1] = BinPoint{(double)q.y, a01.z * kColBytes, a01.w};
-                tile[4 * i4 + 2] = BinPoint{(double)q.z, a23.x * kColBytes, a23.y};
-                tile[4 * i4 + 3] = BinPoint{(double)q.w, a23.z * kColBytes, a23.w};
-            }
-        } else {
-            const uint4* ga = reinterpret_cast<const uint4*>(p.aux32 + cd.off + base);
-            for (uint32_t i4 = tid; i4 < n4; i4 += BLOCK) {
-                const float4 q = gt[i4];
-                const uint4 a = ga[i4];
-                reinterpret_cast<double2*>(tile_t)[2 * i4] = make_double2(q.x, q.y);
-                reinterpret_cast<double2*>(tile_t)[2 * i4 + 1] = make_double2(q.z, q.w);
+        for (uint32_t i4 = tid; i4 < n4; i4 += BLOCK) {
+            float4 q = gt[i4];
+            if constexpr (ALGO == ALGO_AOV) {
+                uint4 a = reinterpret_cast<const uint4*>(p.aux32 + cd.off + base)[i4];
+                // The packed arrays end in zeros; a repeated time with
+                // magnitude 0 keeps the padding out of the edge test of t = 0.
+                if (4 * i4 + 3 >= cnt) {
+                    const float last = src_t[base + cnt - 1];
+                    if (4 * i4 + 1 >= cnt) { q.y = last; a.y = 0u; }
+                    if (4 * i4 + 2 >= cnt) { q.z = last; a.z = 0u; }
+                    if (4 * i4 + 3 >= cnt) { q.w = last; a.w = 0u; }
+                }
                 reinterpret_cast<uint4*>(tile_a)[i4] = a;
             }
+            reinterpret_cast<double2*>(tile_t)[2 * i4] = make_double2(q.x, q.y);
+            reinterpret_cast<double2*>(tile_t)[2 * i4 + 1] = make_double2(q.z, q.w);
         }
     };
     // A curve that fits one tile is staged once for every round.
-    const bool one_tile = n <= kBinTile;
+    const bool one_tile = n_pad <= kBinTile;
     if (one_tile) {
         __syncthreads();
-        stage(0, n);
+        stage(0, n_pad);
         __syncthreads();
     }
 
 #pragma unroll 1
     for (int r = 0; r < ROUNDS; r++) {
-    const uint32_t jr = (uint32_t)(r * BLOCK + tid);
-    const bool active = jr < w.np;
-    const uint32_t pi = w.p0 + (active ? jr : 0u);
-    Cell s;
-    cell_setup<FOLD_EXACT>(s, p.periods[pi], period_dt);
-    const double y32 = s.yhi * 4294967296.0;  // RN(1/P) * 2^32, exact
+    const uint32_t j0 = (uint32_t)(r * CELLS * BLOCK + tid);
+    const bool active = j0 < w.np;  // a thread with any live cell runs all
+    auto cell_period = [&](int c) -> uint32_t {
+        const uint32_t j = j0 + (uint32_t)(c * BLOCK);
+        return w.p0 + (j < w.np ? j : 0u);
+    };
+    // RN(1/P), times 2^32 where the one-FMA bin applies (exact), and pdt / 2P.
+    const double y_scale = fast32 ? 4294967296.0 : 1.0;
+    double ys[CELLS], pc[CELLS];
+#pragma unroll
+    for (int c = 0; c < CELLS; c++) {
+        Cell s;
+        cell_setup<FOLD_EXACT>(s, p.periods[cell_period(c)], period_dt);
+        ys[c] = s.yhi * y_scale;
+        pc[c] = s.c;
+    }
     for (uint32_t k = 0; k < slots; k++)
-        reinterpret_cast<uint32_t*>(cnt_raw)[k * BLOCK + tid] = 0u;
+#pragma unroll
+        for (int c = 0; c < CELLS; c++)
+            reinterpret_cast<uint32_t*>(cnt_raw)[k * kCols + c * BLOCK + tid] = 0u;
 
-    for (uint32_t base = 0; base < n; base += kBinTile) {
-        const uint32_t cnt = min(kBinTile, n - base);
+    uint32_t run_no = 0, run_at = 0, run = 0;  // CE: run number, its first position, its word
+    if constexpr (ALGO == ALGO_CE) run = runs[1];
+
+    for (uint32_t base = 0; base < n_pad; base += kBinTile) {
+        const uint32_t cnt = min(kBinTile, n_pad - base);
         if (!one_tile) {
             __syncthreads();
             stage(base, cnt);
@@ -267,79 +317,64 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
         }
         if (!active) continue;
 
-        // One point: a 128-bit shared load of its record (CE), or its time
-        // and magnitude from the two arrays (AOV).
-        auto load_point = [&](uint32_t i) -> BinPoint {
-            if constexpr (ALGO == ALGO_CE) {
-                const uint4 raw = reinterpret_cast<const uint4*>(tile)[i];
-                return BinPoint{__hiloint2double((int)raw.y, (int)raw.x), raw.z, raw.w};
-            } else {
-                return BinPoint{tile_t[i], tile_a[i], 0u};
-            }
-        };
         // Fast bin of one point: row (+2^31 bias) and the edge-test value
         // ((fraction + D) << 12); the point is near an edge iff ev < edge_lim.
-        auto fast_bin = [&](double td, auto has_pdt_tag, uint32_t& ev) -> uint32_t {
+        auto fast_bin = [&](double td, double y_, double c_, auto has_pdt_tag,
+                            uint32_t& ev) -> uint32_t {
             constexpr bool HAS_PDT = decltype(has_pdt_tag)::value;
-            double a;
-            if constexpr (HAS_PDT) {
-                a = td - s.c * td * td;
-            } else {
-                a = td;
-            }
-            const double qh = __dmul_rn(a, s.yhi);
+            double a = td;
+            if constexpr (HAS_PDT) a = td - c_ * td * td;
+            const double qh = __dmul_rn(a, y_);
             const double r = __dadd_rd(qh, kMagic15);
             const double y = __fma_rd(qh, nd20, kMagic15);
             const uint32_t ylo = (uint32_t)__double2loint(y);
-            const uint32_t yhi = (uint32_t)__double2hiint(y);
+            const uint32_t yup = (uint32_t)__double2hiint(y);
             ev = ylo * 4096u + edge_add;
-            return __funnelshift_r(ylo, yhi, 20) + (uint32_t)__double2loint(r) * n_neg;
+            return __funnelshift_r(ylo, yup, 20) + (uint32_t)__double2loint(r) * n_neg;
         };
-        // |q| < 2^19: y = RD(t_corr * (RN(1/P) * 2^32) + 1.5*2^52), one FMA
-        // on the exact product (closer to t_corr / P than the rounded
+        // |q| < 2^19: y = RD(t_corr * (RN(1/P) * 2^32) + 1.5*2^52 + D), one
+        // FMA on the exact product (closer to t_corr / P than the rounded
         // product fast_bin uses, so the same guard holds), leaves
-        // floor(frac(q') * 2^32) in its low word f.  The 64-bit product
+        // f = floor(frac(q') * 2^32) + D in its low word.  The 64-bit product
         // f * n then holds the row in its high word and the position within
-        // the row in its low word (plus the guard, for the edge test): one
-        // FP64 operation and one integer multiply per point.  The row
-        // carries no bias.
-        auto fast_bin32 = [&](double td, auto has_pdt_tag, uint32_t& ev) -> uint32_t {
+        // the row, D n further on, in its low word: a point within D n of an
+        // edge on either side is one whose low word is below 2 D n, and the
+        // rows of all others are unchanged by D.  One FP64 operation and one
+        // integer multiply per point, and nothing added for the edge test.
+        // The row carries no bias.
+        auto fast_bin32 = [&](double td, double y32, double c_, auto has_pdt_tag,
+                              uint32_t& ev) -> uint32_t {
             constexpr bool HAS_PDT = decltype(has_pdt_tag)::value;
-            double a;
-            if constexpr (HAS_PDT) {
-                a = td - s.c * td * td;
-            } else {
-                a = td;
-            }
-            const double y = __fma_rd(a, y32, kMagic15);
+            double a = td;
+            if constexpr (HAS_PDT) a = td - c_ * td * td;
+            const double y = __fma_rd(a, y32, p.magic32);
             const uint32_t f = (uint32_t)__double2loint(y);
-            const unsigned long long fn = (unsigned long long)f * nP;
-            ev = (uint32_t)fn + edge32_add;
-            return (uint32_t)(fn >> 32);
+            uint32_t row;
+            mul_wide_u32(f, nP, ev, row);
+            return row;
         };
         // The reference's exact sequence (correctly rounded quotient, float
         // fold, f32 divide, then % n_phase: a folded phase of 1.0f gives bin
         // n_phase, which wraps to 0): the bin (+2^31 bias).
-        auto exact_bin = [&](double td, auto has_pdt_tag) -> uint32_t {
+        auto exact_row = [&](double td, const Cell& s, auto has_pdt_tag) -> uint32_t {
             constexpr bool HAS_PDT = decltype(has_pdt_tag)::value;
             const float folded = fold_exact<HAS_PDT>(td, s);
             const uint32_t pb = min(trunc_u(folded / p.phase_bin_size), nP);
             return 0x80000000u + (pb == nP ? 0u : pb);
         };
-        // AOV bytes per bin row, kept opaque to the compiler so that the
-        // counter address is one multiply-add (a power-of-two constant
-        // would become a shift and a separate add).
-        uint32_t aov_row_bytes = 2 * BLOCK * 4;
-        asm("" : "+r"(aov_row_bytes));
-        auto add = [&](uint32_t row, const BinPoint& pt, uint32_t sign) {
-            // sign is 1 (add) or 0xFFFFFFFF (take back); u32 wraparound keeps
-            // packed 16-bit halves and sums exact.
+        // One update: CE adds `inc` to the row's word at `at` (the column's
+        // word of this cell); AOV adds `inc` to the count and `a` to the sum.
+        // The row is kept opaque to the compiler: it would otherwise take
+        // row << k out of the 64-bit product with a funnel shift and a mask,
+        // where a shift-and-add of the high word is one operation.
+        auto add = [&](uint32_t row, uint32_t at, uint32_t inc, uint32_t a) {
+            asm("" : "+r"(row));
             if constexpr (ALGO == ALGO_CE) {
-                red_shared_u32(row * row_stride + pt.a + tbase, pt.b * sign);
+                red_shared_u32(row * (kCols * 4) + at, inc);
             } else {
-                const uint32_t a0 = row * aov_row_bytes + tbase;
-                red_shared_u32(a0, sign);
-                red_shared_u32(a0 + BLOCK * 4, pt.a * sign);
+                const uint32_t a0 = row * (2 * kCols * 4) + at;
+                red_shared_u32(a0, inc);
+                red_shared_u32(a0 + kCols * 4, a);
             }
         };
 
@@ -348,84 +383,148 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
             constexpr bool F32 = decltype(f32_tag)::value;
             // Fast bin (unbiased with F32, +2^31 otherwise; the counter
             // address is the same either way) and its edge limit.
-            auto bin_of = [&](double td, uint32_t& ev) -> uint32_t {
-                if constexpr (F32) return fast_bin32(td, has_pdt_tag, ev);
-                else return fast_bin(td, has_pdt_tag, ev);
+            auto bin_of = [&](double td, double y_, double c_, uint32_t& ev) -> uint32_t {
+                if constexpr (F32) return fast_bin32(td, y_, c_, has_pdt_tag, ev);
+                else return fast_bin(td, y_, c_, has_pdt_tag, ev);
             };
             const uint32_t lim = F32 ? edge32_lim : edge_lim;
-            if constexpr (FAST) {
-                // Groups of 32 points: no branch per point; a group whose
-                // smallest edge-test value is below the limit is revisited
-                // and its near-edge points are moved to the reference's bin.
-                for (uint32_t g = 0; g < cnt; g += 32) {
-                    const uint32_t gend = min(g + 32u, cnt);
-                    uint32_t emin = 0xFFFFFFFFu;
-                    if (gend - g == 32u) {
-                        // A full group unrolled completely: no loop control
-                        // per point (measured 10% faster than unrolling by 4).
-                        // Two running minima of the edge test (even and
-                        // odd points), so the minimum is two short
-                        // dependency chains instead of one of 32 links.
-                        uint32_t emin_b = 0xFFFFFFFFu;
-                        auto one = [&](const BinPoint& pt, uint32_t& em) {
-                            uint32_t ev;
-                            const uint32_t row = bin_of(pt.t, ev);
-                            em = min(em, ev);
-                            add(row, pt, 1u);
-                        };
-                        if constexpr (ALGO == ALGO_CE) {
+            // G staged points from position i, the first `live` of them
+            // real: no branch per point; a group whose smallest edge-test
+            // value is below the limit is revisited and its near-edge
+            // points are moved to the reference's bin.
+            auto group = [&](auto g_tag, auto mask_tag, uint32_t i, uint32_t live, uint32_t at,
+                             uint32_t inc) {
+                constexpr int G = decltype(g_tag)::value;
+                constexpr bool MASK = decltype(mask_tag)::value;
+                double td[G];
+                uint32_t ta[G];
 #pragma unroll
-                            for (uint32_t ii = 0; ii < 32u; ii += 2) {
-                                one(load_point(g + ii), emin);
-                                one(load_point(g + ii + 1), emin_b);
-                            }
-                        } else {
-                            // Four points per two 128-bit loads of times
-                            // and one of magnitudes (g is a multiple of 32).
-                            const double2* t2 = reinterpret_cast<const double2*>(tile_t) + g / 2;
-                            const uint4* a4 = reinterpret_cast<const uint4*>(tile_a) + g / 4;
-#pragma unroll 4
-                            for (uint32_t ii = 0; ii < 8u; ii++) {
-                                const double2 ta = t2[2 * ii], tb = t2[2 * ii + 1];
-                                const uint4 aa = a4[ii];
-                                one(BinPoint{ta.x, aa.x, 0u}, emin);
-                                one(BinPoint{ta.y, aa.y, 0u}, emin_b);
-                                one(BinPoint{tb.x, aa.z, 0u}, emin);
-                                one(BinPoint{tb.y, aa.w, 0u}, emin_b);
-                            }
-                        }
-                        emin = min(emin, emin_b);
-                    } else {
-#pragma unroll 4
-                        for (uint32_t i = g; i < gend; i++) {
-                            const BinPoint pt = load_point(i);
-                            uint32_t ev;
-                            const uint32_t row = bin_of(pt.t, ev);
-                            emin = min(emin, ev);
-                            add(row, pt, 1u);
-                        }
+                for (int k = 0; k < G; k += 2) {
+                    const double2 q = reinterpret_cast<const double2*>(tile_t + i)[k >> 1];
+                    td[k] = q.x;
+                    td[k + 1] = q.y;
+                }
+                if constexpr (ALGO == ALGO_AOV) {
+#pragma unroll
+                    for (int k = 0; k < G; k += 4) {
+                        const uint4 q = reinterpret_cast<const uint4*>(tile_a + i)[k >> 2];
+                        ta[k] = q.x;
+                        ta[k + 1] = q.y;
+                        ta[k + 2] = q.z;
+                        ta[k + 3] = q.w;
                     }
-                    if (emin < lim) {
-                        for (uint32_t i = g; i < gend; i++) {
-                            const BinPoint pt = load_point(i);
+                }
+                uint32_t emin[CELLS];
+#pragma unroll
+                for (int c = 0; c < CELLS; c++) emin[c] = 0xFFFFFFFFu;
+#pragma unroll
+                for (int k = 0; k < G; k++) {
+                    const uint32_t ik = (!MASK || (uint32_t)k < live) ? inc : 0u;
+#pragma unroll
+                    for (int c = 0; c < CELLS; c++) {
+                        uint32_t ev;
+                        const uint32_t row = bin_of(td[k], ys[c], pc[c], ev);
+                        emin[c] = min(emin[c], ev);
+                        add(row, at + c * BLOCK * 4, ik, ALGO == ALGO_AOV ? ta[k] : 0u);
+                    }
+                }
+                uint32_t em = emin[0];
+#pragma unroll
+                for (int c = 1; c < CELLS; c++) em = min(em, emin[c]);
+                if (em < lim) {
+                    // Which of the group's evaluations are near an edge,
+                    // then each of those (rarely more than one).
+                    uint32_t near = 0;
+#pragma unroll
+                    for (int c = 0; c < CELLS; c++)
+#pragma unroll
+                        for (int k = 0; k < G; k++) {
                             uint32_t ev;
-                            const uint32_t row = bin_of(pt.t, ev);
-                            if (ev < lim) {
-                                const uint32_t ex =
-                                    exact_bin(pt.t, has_pdt_tag) - (F32 ? 0x80000000u : 0u);
-                                if (ex != row) {
-                                    add(row, pt, 0xFFFFFFFFu);
-                                    add(ex, pt, 1u);
-                                }
-                            }
+                            bin_of(td[k], ys[c], pc[c], ev);
+                            if (ev < lim) near |= 1u << (c * G + k);
+                        }
+                    if constexpr (MASK) {
+                        const uint32_t m = (1u << live) - 1u;  // 0 < live < G
+#pragma unroll
+                        for (int c = 0; c < CELLS; c++) near &= ~((((1u << G) - 1u) ^ m) << (c * G));
+                    }
+                    while (near) {
+                        const uint32_t e = __ffs(near) - 1;
+                        near &= near - 1;
+                        const uint32_t c = e / G, k = e % G;
+                        Cell s;
+                        cell_setup<FOLD_EXACT>(s, p.periods[cell_period(c)], period_dt);
+                        const double t = tile_t[i + k];
+                        uint32_t ev;
+                        const uint32_t row = bin_of(t, s.yhi * y_scale, s.c, ev);
+                        const uint32_t ex =
+                            exact_row(t, s, has_pdt_tag) - (F32 ? 0x80000000u : 0u);
+                        if (ex != row) {
+                            // u32 wraparound keeps packed halves and sums exact.
+                            const uint32_t a = ALGO == ALGO_AOV ? tile_a[i + k] : 0u;
+                            add(row, at + c * BLOCK * 4, 0u - inc, 0u - a);
+                            add(ex, at + c * BLOCK * 4, inc, a);
                         }
                     }
                 }
+            };
+            // m points from tile position i (a multiple of 4).
+            auto span = [&](uint32_t i, uint32_t m, uint32_t at, uint32_t inc) {
+                if constexpr (FAST) {
+                    // Groups of 16 (CE; 16 were slower for AOV, whose two
+                    // reductions per point need the registers), then 8, 4
+                    // and the rest of the last four.
+                    using G16 = std::integral_constant<int, 16>;
+                    using G8 = std::integral_constant<int, 8>;
+                    using G4 = std::integral_constant<int, 4>;
+                    using Whole = std::false_type;
+                    uint32_t k = 0;
+                    if constexpr (ALGO == ALGO_CE) {
+#pragma unroll 1
+                        for (; k + 16 <= m; k += 16) group(G16{}, Whole{}, i + k, 16u, at, inc);
+                        if (k + 8 <= m) {
+                            group(G8{}, Whole{}, i + k, 8u, at, inc);
+                            k += 8;
+                        }
+                    } else {
+#pragma unroll 1
+                        for (; k + 8 <= m; k += 8) group(G8{}, Whole{}, i + k, 8u, at, inc);
+                    }
+                    if (k + 4 <= m) {
+                        group(G4{}, Whole{}, i + k, 4u, at, inc);
+                        k += 4;
+                    }
+                    if (k < m) group(G4{}, std::true_type{}, i + k, m - k, at, inc);
+                } else {
+#pragma unroll 1
+                    for (int c = 0; c < CELLS; c++) {
+                        Cell s;
+                        cell_setup<FOLD_EXACT>(s, p.periods[cell_period(c)], period_dt);
+#pragma unroll 2
+                        for (uint32_t k = 0; k < m; k++)
+                            add(exact_row(tile_t[i + k], s, has_pdt_tag), at + c * BLOCK * 4, inc,
+                                ALGO == ALGO_AOV ? tile_a[i + k] : 0u);
+                    }
+                }
+            };
+            if constexpr (ALGO == ALGO_AOV) {
+                span(0u, cnt, tbase, 1u);
             } else {
-#pragma unroll 4
-                for (uint32_t i = 0; i < cnt; i++) {
-                    const BinPoint pt = load_point(i);
-                    add(exact_bin(pt.t, has_pdt_tag), pt, 1u);
+                // The runs (one magnitude column each) that meet this tile.
+                const uint32_t end = base + cnt;
+                while (run != 0u && run_at < end) {
+                    const uint32_t len = run & 0xFFFFu, col = run >> 16;
+                    const uint32_t lo = max(run_at, base), hi = min(run_at + len, end);
+                    const uint32_t next = runs[run_no + 2];
+                    const uint32_t word = CNT16 ? col >> 1 : col;
+                    if (hi > lo)
+                        span(lo - base, hi - lo, tbase + word * (nP * kCols * 4),
+                             (CNT16 && (col & 1u)) ? 0x10000u : 1u);
+                    const uint32_t next_at = run_at + ((len + 3u) & ~3u);
+                    if (next_at > end) break;  // the rest lies in the next tile
+                    run_at = next_at;
+                    run = next;
+                    run_no++;
                 }
             }
         };
@@ -445,22 +544,26 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
     // statistic after it).
     compiler_fence();
     __syncwarp();
-    if (active) {
+#pragma unroll 1
+    for (int c = 0; c < CELLS; c++) {
+    const uint32_t pi = cell_period(c);
+    if (j0 + (uint32_t)(c * BLOCK) < w.np) {
     const size_t out_idx =
         (size_t)w.curve * ((size_t)p.n_per * p.n_pdt) + (size_t)pi * p.n_pdt + w.pdt;
-    uint32_t* cnt32 = reinterpret_cast<uint32_t*>(cnt_raw);
+    const uint32_t* cnt32 = reinterpret_cast<const uint32_t*>(cnt_raw) + c * BLOCK;
+    const uint32_t cbase = tbase + c * BLOCK * 4;
 
     if constexpr (ALGO == ALGO_CE && !REF_STATS) {
-        p.out[out_idx] = ce_stat_fast<CNT16>(tbase, nP, W, BLOCK, n);
+        p.out[out_idx] = ce_stat_fast<CNT16>(cbase, nP, W, kCols, n);
     } else if constexpr (ALGO == ALGO_AOV && !REF_STATS) {
-        p.out[out_idx] = aov_finish(aov_sbx_fast(tbase, nP, BLOCK), cd, n, nP);
+        p.out[out_idx] = aov_finish(aov_sbx_fast(cbase, nP, kCols), cd, n, nP);
     } else if constexpr (ALGO == ALGO_CE) {
         auto count = [&](uint32_t j, uint32_t i) -> uint32_t {
             if constexpr (CNT16) {
-                const uint32_t wv = cnt32[(j * W + (i >> 1)) * BLOCK + tid];
+                const uint32_t wv = cnt32[((i >> 1) * nP + j) * kCols + tid];
                 return (i & 1u) ? (wv >> 16) : (wv & 0xFFFFu);
             } else {
-                return cnt32[(j * W + i) * BLOCK + tid];
+                return cnt32[(i * nP + j) * kCols + tid];
             }
         };
         if (p.bins) {
@@ -489,16 +592,16 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
         }
         p.out[out_idx] = ce;
     } else {
-        const uint32_t* sums = cnt32 + BLOCK;
+        const uint32_t* sums = cnt32 + kCols;
         if (p.bins) {
             uint32_t* o = p.bins + out_idx * (size_t)nP;
-            for (uint32_t b = 0; b < nP; b++) o[b] = cnt32[2 * b * BLOCK + tid];
+            for (uint32_t b = 0; b < nP; b++) o[b] = cnt32[2 * b * kCols + tid];
         }
         const double xbar = cd.fix_sumx / (double)n;
         double s1 = 0.0, sbx = 0.0;
         for (uint32_t b = 0; b < nP; b++) {
-            const uint32_t c = cnt32[2 * b * BLOCK + tid];
-            const uint32_t X = sums[2 * b * BLOCK + tid];
+            const uint32_t c = cnt32[2 * b * kCols + tid];
+            const uint32_t X = sums[2 * b * kCols + tid];
             if (c != 0u) {
                 const double nb = (double)c;
                 const double Xd = (double)X;
@@ -516,33 +619,79 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
         p.out[out_idx] = (float)(scale * (s1 / (s2 <= 0.0 ? 0.0 : s2)));
 #endif
     }
-    }  // active
+    }  // a live cell
+    }  // cells
     }  // rounds
     stamp_end(p, item);
 }
 
-// Items from the device work queue (see WorkQueue), persistently or one CTA
-// per item; an item is ROUNDS x BLOCK consecutive periods.
-template <int ALGO, bool CNT16, int BLOCK, bool REF_STATS, bool PERSIST, int ROUNDS>
-__global__ void __launch_bounds__(BLOCK, queue_min_blocks<ALGO, BLOCK>())
+// One CTA per item of the device work queue (see WorkQueue); an item is
+// ROUNDS x CELLS x BLOCK consecutive periods.  (Persistent CTAs measured 1-8%
+// slower in every class.)
+template <int ALGO, bool CNT16, int BLOCK, bool REF_STATS, int ROUNDS, int CELLS>
+__global__ void __launch_bounds__(BLOCK, bin_min_blocks<ALGO, BLOCK, CELLS>())
     bin_kernel(const FoldParams p) {
-    if constexpr (PERSIST) {
-        for_each_queued_item<BLOCK * ROUNDS>(p, [&](const WorkItem& w, uint32_t k) {
-            bin_item<ALGO, CNT16, BLOCK, REF_STATS, ROUNDS>(p, w, k);
-        });
-    } else {
-        bin_item<ALGO, CNT16, BLOCK, REF_STATS, ROUNDS>(
-            p, queue_item<BLOCK * ROUNDS>(p, blockIdx.x), blockIdx.x);
+    bin_item<ALGO, CNT16, BLOCK, REF_STATS, ROUNDS, CELLS>(
+        p, queue_item<BLOCK * ROUNDS * CELLS>(p, blockIdx.x), blockIdx.x);
+}
+
+// CE times sorted by magnitude column, for bin_kernel: equal columns lie
+// together, so the kernel keeps a column's counter address and increment in
+// registers for the whole run and a staged point is its time alone (8 bytes
+// instead of a 16-byte record).  Counts do not depend on the order.  Per
+// curve: ts = the runs one after the other, each padded to a multiple of 4
+// with repeats of its first time; runs = {padded total, then one word
+// (column << 16) | length per non-empty column, then 0}.
+__global__ void __launch_bounds__(256)
+    ce_sort_kernel(const float* __restrict__ t, const float* __restrict__ m,
+                   const CurveDesc* __restrict__ curves, uint32_t n_curves, uint32_t n_mag,
+                   float mag_bin_size, CeSortLayout lay, float* __restrict__ ts,
+                   uint32_t* __restrict__ runs) {
+    extern __shared__ uint32_t sort_cnt[];  // [n_mag] counts, [n_mag] write positions
+    uint32_t* sort_pos = sort_cnt + n_mag;
+    const uint32_t c = blockIdx.x;
+    if (c >= n_curves) return;
+    const CurveDesc cd = curves[c];
+    float* tc = ts + (cd.off * lay.ts_mul + (int64_t)c * lay.ts_pad);
+    uint32_t* rc = runs + (cd.off * lay.run_mul + (int64_t)c * lay.run_pad);
+    // MagBin (periodfind/cuda/ce.cu:70-72; rust/src/ce.rs:79).
+    auto column = [&](uint32_t i) -> uint32_t {
+        const unsigned long long mb64 =
+            static_cast<unsigned long long>(m[cd.off + i] / mag_bin_size);
+        return (uint32_t)(mb64 % n_mag);
+    };
+    for (uint32_t k = threadIdx.x; k < n_mag; k += 256) sort_cnt[k] = 0u;
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < cd.n; i += 256) atomicAdd(&sort_cnt[column(i)], 1u);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t at = 0, r = 0;
+        for (uint32_t k = 0; k < n_mag; k++) {
+            const uint32_t len = sort_cnt[k];
+            sort_pos[k] = at;
+            if (len) rc[1 + r++] = (k << 16) | len;
+            at += (len + 3u) & ~3u;
+        }
+        rc[1 + r] = 0u;
+        rc[0] = at;
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < cd.n; i += 256)
+        tc[atomicAdd(&sort_pos[column(i)], 1u)] = t[cd.off + i];
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < n_mag; k += 256) {
+        const uint32_t len = sort_cnt[k], end = sort_pos[k];
+        if (!len) continue;
+        const float first = tc[end - len];
+        for (uint32_t e = end; e < end - len + ((len + 3u) & ~3u); e++) tc[e] = first;
     }
 }
 
-// CE per-point bin data for bin_kernel: {counter word of the magnitude
-// column within a phase row, increment}.  The kernel turns the word into a
-// byte offset for its CTA shape when it stages the tile, so the data serves
-// every block size the autotuner tries.
+// CE per-point bin data of the shared-histogram kernel (pf_binwarp.cuh):
+// {16-bit counter word of the magnitude column, increment}.
 __global__ void ce_binaux_kernel(const float* __restrict__ m, uint2* __restrict__ aux,
                                  const CurveDesc* __restrict__ curves, uint32_t n_curves,
-                                 uint32_t n_mag, float mag_bin_size, int cnt16) {
+                                 uint32_t n_mag, float mag_bin_size) {
     const uint32_t c = blockIdx.x;
     if (c >= n_curves) return;
     const CurveDesc cd = curves[c];
@@ -550,18 +699,12 @@ __global__ void ce_binaux_kernel(const float* __restrict__ m, uint2* __restrict_
     for (uint32_t i = threadIdx.x; i < n4; i += blockDim.x) {
         uint2 v = make_uint2(0u, 0u);
         if (i < cd.n) {
-            const float mag_val = m[cd.off + i];
             // MagBin (periodfind/cuda/ce.cu:70-72; rust/src/ce.rs:79).
             const unsigned long long mb64 =
-                static_cast<unsigned long long>(mag_val / mag_bin_size);
+                static_cast<unsigned long long>(m[cd.off + i] / mag_bin_size);
             const uint32_t mb = (uint32_t)(mb64 % n_mag);
-            if (cnt16) {
-                v.x = mb >> 1;
-                v.y = (mb & 1u) ? 0x10000u : 1u;
-            } else {
-                v.x = mb;
-                v.y = 1u;
-            }
+            v.x = mb >> 1;
+            v.y = (mb & 1u) ? 0x10000u : 1u;
         }
         aux[cd.off + i] = v;
     }

@@ -248,13 +248,12 @@ __device__ __forceinline__ void for_each_queued_item(const FoldParams& p, F&& f)
     }
 }
 
-// Resident CTAs per SM the queue kernels are compiled for (registers held
-// so that occupancy is not lost to the register allocator; measured): the LS
-// folds and the AOV bin kernel at 5 x 256 threads, the CE bin kernel at its
-// shared-memory limit of 4 x 256 (CE 10 x 10).
-template <int ALGO, int BLOCK>
+// Resident CTAs per SM the LS folds are compiled for (registers held so that
+// occupancy is not lost to the register allocator; measured): 5 x 256
+// threads.
+template <int BLOCK>
 constexpr int queue_min_blocks() {
-    return (ALGO == ALGO_CE ? 4 : 5) * 256 / BLOCK;
+    return 5 * 256 / BLOCK;
 }
 
 // trunc(q) for finite q in [0, 2^23): identical to the reference's
@@ -647,7 +646,7 @@ __device__ __forceinline__ void fold_item(const FoldParams& p, const WorkItem w,
 // the reference launches.
 template <int ALGO, int FOLD, int ACC, int BLOCK, bool OVL, bool PERSIST>
 __global__ void __launch_bounds__(BLOCK, (ALGO == ALGO_LS && uses_queue(KIND_FOLD, FOLD))
-                                             ? queue_min_blocks<ALGO_LS, BLOCK>()
+                                             ? queue_min_blocks<BLOCK>()
                                              : 1)
     fold_kernel(const FoldParams p) {
     if constexpr (!uses_queue(KIND_FOLD, FOLD)) {

@@ -37,9 +37,11 @@ struct FoldConfig {
     int block;  // threads per CTA: 64, 128 or 256
     bool ovl;   // general bin-overlap path
     bool ref_stats; // bin_kernel: the reference's statistic operation sequence
-    bool persist;   // queue kernels: persistent grid instead of one CTA per item
-    int rounds;     // bin kernel: an item is rounds x block periods (1 or 4);
+    bool persist;   // queue kernels but the bin kernel: persistent grid instead of
+                    // one CTA per item
+    int rounds;     // bin kernel: an item is rounds x cells x block periods (1 or 4);
                     // KIND_LSREC: frequencies per thread (4 or 8)
+    int cells;      // bin kernel: periods a thread holds at once (1 or 2)
     int n_sm;       // persistent kernels: grid = n_sm x resident CTAs per SM
 };
 
@@ -47,7 +49,10 @@ size_t fold_smem(const FoldConfig& c, uint32_t n_phase, uint32_t n_mag);
 
 // Periods in one work item of a queue kernel.
 inline int item_periods(const FoldConfig& c) {
-    return c.block * ((c.kind == KIND_BIN || c.kind == KIND_LSREC) && c.rounds > 1 ? c.rounds : 1);
+    int n = c.block;
+    if ((c.kind == KIND_BIN || c.kind == KIND_LSREC) && c.rounds > 1) n *= c.rounds;
+    if (c.kind == KIND_BIN && c.cells > 1) n *= c.cells;
+    return n;
 }
 
 // Semantics of the reference's CUDA build (-use_fast_math).
@@ -65,10 +70,18 @@ cudaError_t launch_magbin_cpusem(const float* m, uint32_t* aux, const CurveDesc*
 
 cudaError_t launch_binaux_cudasem(const float* m, void* aux, const CurveDesc* curves,
                                   uint32_t n_curves, uint32_t n_mag, float mag_bin_size,
-                                  int block, int cnt16, cudaStream_t s);
+                                  cudaStream_t s);
+cudaError_t launch_cesort_cudasem(const float* t, const float* m, const CurveDesc* curves,
+                                  uint32_t n_curves, uint32_t n_mag, float mag_bin_size,
+                                  const CeSortLayout& lay, float* ts, uint32_t* runs,
+                                  cudaStream_t s);
 cudaError_t launch_binaux_cpusem(const float* m, void* aux, const CurveDesc* curves,
-                                 uint32_t n_curves, uint32_t n_mag, float mag_bin_size,
-                                 int block, int cnt16, cudaStream_t s);
+                                  uint32_t n_curves, uint32_t n_mag, float mag_bin_size,
+                                  cudaStream_t s);
+cudaError_t launch_cesort_cpusem(const float* t, const float* m, const CurveDesc* curves,
+                                  uint32_t n_curves, uint32_t n_mag, float mag_bin_size,
+                                  const CeSortLayout& lay, float* ts, uint32_t* runs,
+                                  cudaStream_t s);
 
 // FPW and BLS (pf_fpw.cuh): per point t, inverse variance iv = 1 / err^2 and
 // ivy = iv * m, packed per curve at off[c] with len[c] points; out is

@@ -59,11 +59,21 @@ struct WorkQueue {
     unsigned* next;
 };
 
+// Where a curve's sorted CE times and run table start (pf_bin.cuh,
+// ce_sort_kernel): off * mul + curve * pad.
+struct CeSortLayout {
+    uint32_t ts_mul, ts_pad;    // floats
+    uint32_t run_mul, run_pad;  // words
+};
+
 struct FoldParams {
     const float* t;          // packed times
     const float* m;          // packed magnitudes (AOV F32, LS)
     const uint32_t* aux32;   // CE: packed magnitude bin per point
     const uint64_t* aux64;   // AOV FIX: packed (1 << 44) + fixed-point mag
+    const float* ts;         // CE bin kernel: times sorted by magnitude column
+    const uint32_t* runs;    // CE bin kernel: the columns' runs
+    uint32_t ts_mul, ts_pad, run_mul, run_pad;  // their CeSortLayout
     const CurveDesc* curves;
     const WorkItem* work;
     const float* periods;
@@ -74,6 +84,11 @@ struct FoldParams {
     float phase_bin_size, mag_bin_size;
     const unsigned* tmax_bits;  // float bits of max |t| over the batch
     uint32_t edge_d;            // bin-edge guard (units of 2^-20 of a bin)
+    // One-FMA bin (pf_bin.cuh, fast_bin32): 1.5 * 2^52 + D and the edge limit
+    // 2 D n_phase, with D n_phase at least the guard in units of 2^-32 of a
+    // bin plus n_phase for the truncation of the phase to 32 bits.
+    double magic32;
+    uint32_t edge32_lim;
     unsigned long long* stamps; // optional: [work item][start, end] globaltimer ns
     WorkQueue q;                // persistent kernels (instead of `work`)
     // Optional (occupancy tests): raw bin counts per cell, [curve][n_per]
@@ -87,15 +102,22 @@ struct FoldParams {
     double f0, df;
 };
 
-// Shared-memory bytes of the chosen bin kernel (pf_bin.cuh).
-inline size_t bin_smem_bytes(int algo, bool cnt16, int block, uint32_t n_phase,
+// Staged points of the chosen bin kernel: the time as a double, for AOV also
+// the fixed-point magnitude.
+__host__ __device__ constexpr size_t bin_tile_bytes(int algo) {
+    return (size_t)kBinTile * (algo == ALGO_CE ? 8 : 12);
+}
+
+// Shared-memory bytes of the chosen bin kernel (pf_bin.cuh); cols = periods
+// held by the CTA at once (threads x cells per thread).
+inline size_t bin_smem_bytes(int algo, bool cnt16, int cols, uint32_t n_phase,
                              uint32_t n_mag) {
-    size_t bytes = (size_t)kBinTile * 16;  // {double t; u32 a, b} per point
+    size_t bytes = bin_tile_bytes(algo);
     if (algo == ALGO_CE) {
         const size_t w = cnt16 ? (n_mag + 1) / 2 : n_mag;
-        bytes += (size_t)n_phase * w * block * 4;
+        bytes += (size_t)n_phase * w * cols * 4;
     } else {
-        bytes += (size_t)2 * n_phase * block * 4;
+        bytes += (size_t)2 * n_phase * cols * 4;
     }
     return bytes;
 }
