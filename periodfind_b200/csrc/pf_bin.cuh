@@ -49,8 +49,9 @@
 //     three-way minimum (6.4 instructions with all overheads on 4096 points,
 //     11.1 before).
 // Measured, 3000 ragged curves (20-2000 points) x 20000 periods, CE 10 x 10
-// then AOV 15, plan with peaks: 12.06 -> 10.50 ms and 11.63 -> 9.05 ms;
-// CE 200 x 4096 x 10000 x 2 derivatives 7.26 -> 5.27 ms.  CE [1024,4096):
+// then AOV 15, plan with peaks: 12.06 -> 10.40 ms and 11.63 -> 8.99 ms (9.57
+// and 8.86 ms with the statistics below); CE 200 x 4096 x 10000 x 2
+// derivatives 7.26 -> 5.18 ms.  CE [1024,4096):
 // issue 61%, fmaheavy pipe 73%, shared-memory pipe 50%; AOV: shared-memory
 // pipe 88% (its two reductions per evaluation).
 #pragma once
@@ -117,12 +118,18 @@ __device__ __forceinline__ float ce_finish(float acc, uint32_t n) {
     return __fmul_rn(acc, 0.69314718055994531f / (float)n);
 }
 
-// AOV of one cell from sum_b X_b^2 / c_b (fixed-point bin sums X_b).
-__device__ __forceinline__ float aov_finish(double sbx, const CurveDesc& cd, uint32_t n,
-                                            uint32_t nP) {
-    const double s1 = fmax(sbx - cd.fix_sumx * cd.fix_sumx / (double)n, 0.0);
-    const double s2 = __dadd_rn(cd.fix_sumx2, -sbx);
-    const double scale = ((double)n - (double)nP) / ((double)nP - 1.0);
+// AOV of one cell from sum_b X_b^2 / c_b (fixed-point bin sums X_b); per
+// curve, xx_n = X^2 / n and scale = (n - nP) / (nP - 1).
+__device__ __forceinline__ double aov_xx_n(const CurveDesc& cd) {
+    return cd.fix_sumx * cd.fix_sumx / (double)cd.n;
+}
+__device__ __forceinline__ double aov_scale(uint32_t n, uint32_t nP) {
+    return ((double)n - (double)nP) / ((double)nP - 1.0);
+}
+__device__ __forceinline__ float aov_finish(double sbx, double xx_n, double sumx2,
+                                            double scale) {
+    const double s1 = fmax(sbx - xx_n, 0.0);
+    const double s2 = __dadd_rn(sumx2, -sbx);
 #if PF_SEM_CPU_TU
     return (s2 <= 0.0) ? 0.0f : (float)(scale * (s1 / s2));
 #else
@@ -130,49 +137,107 @@ __device__ __forceinline__ float aov_finish(double sbx, const CurveDesc& cd, uin
 #endif
 }
 
-// The chosen form's CE statistic.  Counters are read through 32-bit shared
-// addresses (tbase = this thread's column).  Each row term
+// The chosen form's CE statistic of CELLS cells at once.  Counters are read
+// through 32-bit shared addresses (tbase = the thread's first column, the
+// cells cell_bytes apart).  Each row term
 // C_j ln C_j - sum_i c_ij ln c_ij is non-negative, so FP32 accumulation keeps
 // the relative error near 1e-7 (FP64 here costs registers in the binning
 // loop, measured slower).  Per row, the magnitude bins are taken in pairs
-// (the two 16-bit halves of a word).
-template <bool CNT16>
-__device__ __forceinline__ float ce_stat_fast(uint32_t tbase, uint32_t nP, uint32_t W,
-                                              uint32_t block, uint32_t n) {
-    auto xlx = [](uint32_t c) -> float { return ce_xlx(c); };
-    float acc = 0.0f;
-    for (uint32_t j = 0; j < nP; j++) {
-        uint32_t col = 0;
-        float row = 0.0f;
-        for (uint32_t wi = 0; wi < W; wi++) {
-            const uint32_t wv = lds_u32(tbase + (wi * nP + j) * block * 4u);
-            if constexpr (CNT16) {
-                // Both 16-bit halves summed at once: each half's column
-                // total is at most n < 2^16, so no carry crosses halves.
-                col += wv;
-                row = __fadd_rn(row, __fadd_rn(xlx(wv & 0xFFFFu), xlx(wv >> 16)));
-            } else {
-                col += wv;
-                row = __fadd_rn(row, xlx(wv));
+// (the two 16-bit halves of a word).  A cell's sum is one long chain of
+// loads, logs and adds, so two rows of every cell run side by side (tuning
+// samples of 10 x 10 bins, one cell and row at a time -> this: [64,256) 1.31
+// -> 1.15 ms, [256,1024) 0.76 -> 0.70, [1024,4096) 0.60 -> 0.57; the floor is
+// the log's 110 operations per cell on the XU pipe).  8-bit counters for
+// curves under 256 points, which double the resident warps, were slower
+// (1.15 -> 1.18 ms).
+template <bool CNT16, int CELLS>
+__device__ __forceinline__ void ce_stat_fast(uint32_t tbase, uint32_t cell_bytes, uint32_t nP,
+                                             uint32_t W, uint32_t cols, uint32_t n,
+                                             float (&out)[CELLS]) {
+    float acc[CELLS];
+#pragma unroll
+    for (int c = 0; c < CELLS; c++) acc[c] = 0.0f;
+    auto rows = [&](auto rows_tag, uint32_t j) {
+        constexpr int R = decltype(rows_tag)::value;
+        uint32_t col[R][CELLS];
+        float row[R][CELLS];
+#pragma unroll
+        for (int r = 0; r < R; r++)
+#pragma unroll
+            for (int c = 0; c < CELLS; c++) {
+                col[r][c] = 0u;
+                row[r][c] = 0.0f;
             }
+        uint32_t at = tbase + j * (cols * 4u);
+#pragma unroll 1
+        for (uint32_t wi = 0; wi < W; wi++, at += nP * (cols * 4u)) {
+#pragma unroll
+            for (int r = 0; r < R; r++)
+#pragma unroll
+                for (int c = 0; c < CELLS; c++) {
+                    const uint32_t wv = lds_u32(at + r * (cols * 4u) + c * cell_bytes);
+                    // Both 16-bit halves summed at once: each half's total
+                    // is at most n < 2^16, so no carry crosses halves.
+                    col[r][c] += wv;
+                    row[r][c] = __fadd_rn(
+                        row[r][c], CNT16 ? __fadd_rn(ce_xlx(wv & 0xFFFFu), ce_xlx(wv >> 16))
+                                         : ce_xlx(wv));
+                }
         }
-        if constexpr (CNT16) col = (col & 0xFFFFu) + (col >> 16);
-        acc = __fadd_rn(acc, __fsub_rn(xlx(col), row));
-    }
-    return ce_finish(acc, n);
+#pragma unroll
+        for (int r = 0; r < R; r++)
+#pragma unroll
+            for (int c = 0; c < CELLS; c++) {
+                const uint32_t t = CNT16 ? (col[r][c] & 0xFFFFu) + (col[r][c] >> 16) : col[r][c];
+                acc[c] = __fadd_rn(acc[c], __fsub_rn(ce_xlx(t), row[r][c]));
+            }
+    };
+    uint32_t j = 0;
+#pragma unroll 1
+    for (; j + 2 <= nP; j += 2) rows(std::integral_constant<int, 2>{}, j);
+    if (j < nP) rows(std::integral_constant<int, 1>{}, j);
+#pragma unroll
+    for (int c = 0; c < CELLS; c++) out[c] = ce_finish(acc[c], n);
+}
+
+// An unsigned integer as a double: placed in the mantissa of 2^52, which is
+// then taken off (exact, and no conversion instruction).
+__device__ __forceinline__ double u32_to_double(uint32_t v) {
+    return __dadd_rn(__hiloint2double(0x43300000, (int)v), -4503599627370496.0);
+}
+
+// 1 / c rounded to nearest for a count 1 <= c < 65536: two Newton steps
+// r += r (1 - c r) from the hardware's approximation.  With a start good to
+// 2^-18 the second step's error is below 2^-70 of the result, and 1 / c for
+// c < 2^16 lies at least 2^-70 from every midpoint of two doubles, so the
+// last rounding is the right one (checked against __drcp_rn for every c).
+__device__ __forceinline__ double count_rcp(uint32_t c) {
+    const double x = u32_to_double(c);
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    r = __fma_rn(r, __fma_rn(-x, r, 1.0), r);
+    return __fma_rn(r, __fma_rn(-x, r, 1.0), r);
 }
 
 // The chosen form's AOV sum_b X_b^2 / c_b over the fixed-point bin sums X_b
-// (empty bins have X_b = 0 and contribute nothing).  Counters [bin][count,
-// sum][thread].
-__device__ __forceinline__ double aov_sbx_fast(uint32_t tbase, uint32_t nP, uint32_t block) {
-    double sbx = 0.0;
+// (empty bins have X_b = 0 and contribute nothing), CELLS cells at once
+// ([64,256) samples 0.87 -> 0.81 ms against library reciprocals and integer
+// conversions).  Counters [bin][count, sum][cols].
+template <int CELLS>
+__device__ __forceinline__ void aov_sbx_fast(uint32_t tbase, uint32_t cell_bytes, uint32_t nP,
+                                             uint32_t cols, double (&sbx)[CELLS]) {
+#pragma unroll
+    for (int c = 0; c < CELLS; c++) sbx[c] = 0.0;
+#pragma unroll 2
     for (uint32_t b = 0; b < nP; b++) {
-        const uint32_t c = lds_u32(tbase + 2u * b * block * 4u);
-        const double Xd = (double)lds_u32(tbase + (2u * b + 1u) * block * 4u);
-        sbx = __fma_rn(__dmul_rn(Xd, Xd), __drcp_rn((double)max(c, 1u)), sbx);
+#pragma unroll
+        for (int c = 0; c < CELLS; c++) {
+            const uint32_t at = tbase + b * (2u * cols * 4u) + c * cell_bytes;
+            const uint32_t cnt = lds_u32(at);
+            const double Xd = u32_to_double(lds_u32(at + cols * 4u));
+            sbx[c] = __fma_rn(__dmul_rn(Xd, Xd), count_rcp(max(cnt, 1u)), sbx[c]);
+        }
     }
-    return sbx;
 }
 
 // Statistic forms.  REF_STATS: the reference's operation sequence
@@ -230,6 +295,12 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
         my_pmin = fmin(my_pmin, fabs((double)per));
     }
     const double qb = cta_qbound_of<BLOCK>(p, my_pmin, period_dt);
+    // The two FP64 divides of the AOV statistic that depend on the curve only.
+    __shared__ double s_aov[2];
+    if (ALGO == ALGO_AOV && !REF_STATS && tid == 0) {
+        s_aov[0] = aov_xx_n(cd);
+        s_aov[1] = aov_scale(n, nP);
+    }
     const bool fast = __syncthreads_and(fin ? 1 : 0) && qb * (double)nP < 1073741824.0;  // 2^30
     // |q| < 2^19 as well: the phase's 32 fraction bits come from one FMA.
     const bool fast32 = fast && qb < 524288.0;
@@ -544,20 +615,33 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
     // statistic after it).
     compiler_fence();
     __syncwarp();
-#pragma unroll 1
-    for (int c = 0; c < CELLS; c++) {
-    const uint32_t pi = cell_period(c);
-    if (j0 + (uint32_t)(c * BLOCK) < w.np) {
+    if constexpr (!REF_STATS) {
+        if (active) {
+            float res[CELLS];
+            if constexpr (ALGO == ALGO_CE) {
+                ce_stat_fast<CNT16, CELLS>(tbase, BLOCK * 4, nP, W, kCols, n, res);
+            } else {
+                double sbx[CELLS];
+                aov_sbx_fast<CELLS>(tbase, BLOCK * 4, nP, kCols, sbx);
+#pragma unroll
+                for (int c = 0; c < CELLS; c++)
+                    res[c] = aov_finish(sbx[c], s_aov[0], cd.fix_sumx2, s_aov[1]);
+            }
+#pragma unroll
+            for (int c = 0; c < CELLS; c++)
+                if (j0 + (uint32_t)(c * BLOCK) < w.np)
+                    p.out[(size_t)w.curve * ((size_t)p.n_per * p.n_pdt) +
+                          (size_t)cell_period(c) * p.n_pdt + w.pdt] = res[c];
+        }
+        continue;
+    }
+    // The reference statistic (one cell per thread).
+    if (active) {
+    const uint32_t pi = cell_period(0);
     const size_t out_idx =
         (size_t)w.curve * ((size_t)p.n_per * p.n_pdt) + (size_t)pi * p.n_pdt + w.pdt;
-    const uint32_t* cnt32 = reinterpret_cast<const uint32_t*>(cnt_raw) + c * BLOCK;
-    const uint32_t cbase = tbase + c * BLOCK * 4;
-
-    if constexpr (ALGO == ALGO_CE && !REF_STATS) {
-        p.out[out_idx] = ce_stat_fast<CNT16>(cbase, nP, W, kCols, n);
-    } else if constexpr (ALGO == ALGO_AOV && !REF_STATS) {
-        p.out[out_idx] = aov_finish(aov_sbx_fast(cbase, nP, kCols), cd, n, nP);
-    } else if constexpr (ALGO == ALGO_CE) {
+    const uint32_t* cnt32 = reinterpret_cast<const uint32_t*>(cnt_raw);
+    if constexpr (ALGO == ALGO_CE) {
         auto count = [&](uint32_t j, uint32_t i) -> uint32_t {
             if constexpr (CNT16) {
                 const uint32_t wv = cnt32[((i >> 1) * nP + j) * kCols + tid];
@@ -620,7 +704,6 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
 #endif
     }
     }  // a live cell
-    }  // cells
     }  // rounds
     stamp_end(p, item);
 }

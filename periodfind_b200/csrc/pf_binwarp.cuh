@@ -175,7 +175,9 @@ __device__ __forceinline__ void binwarp_item(const FoldParams& p, const WorkItem
                     sbx = __fma_rn(__shfl_sync(0xffffffffu, x2, (int)l),
                                    __shfl_sync(0xffffffffu, rc, (int)l), sbx);
             }
-            if (lane == 0) p.out[out_idx] = aov_finish(sbx, cd, n, nP);
+            if (lane == 0)
+                p.out[out_idx] =
+                    aov_finish(sbx, aov_xx_n(cd), cd.fix_sumx2, aov_scale(n, nP));
         }
         __syncwarp();
     }
