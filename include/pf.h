@@ -64,11 +64,14 @@
  *                  pending on a context; a third is PF_EINVAL.  A caller
  *                  packs the next batch while the GPU runs this one.  Not
  *                  with PF_TIMING.
- *  PF_TRIG_SINCOS / PF_TRIG_RECURRENCE  (pf_ls_fgrid*, chosen) keep one trig
+ *  PF_TRIG_SINCOS / PF_TRIG_RECURRENCE / PF_TRIG_TRANSFORM  (pf_ls_fgrid*,
+ *                  chosen) keep one trig
  *                  form instead of letting the autotuner pick per length
- *                  class: MUFU sine / cosine at every (point, frequency), or
+ *                  class: MUFU sine / cosine at every (point, frequency),
  *                  one sine / cosine per point and thread followed by
- *                  angle-addition rotations along the uniform grid.
+ *                  angle-addition rotations along the uniform grid, or a
+ *                  non-uniform FFT of the points (blocks of 4096
+ *                  frequencies; a candidate from 1024 frequencies on).
  *  PF_BINS_SHARED  (CE / AOV, chosen) keep the shared-histogram binning
  *                  (one histogram per warp and trial period, filled with
  *                  shared atomics) for the length classes it serves (curves
@@ -116,6 +119,7 @@ extern "C" {
 #define PF_ONE_LAUNCH 0x80000
 #define PF_HOST_NORMALIZE 0x100000
 #define PF_HOST_CENTER 0x200000
+#define PF_TRIG_TRANSFORM 0x400000
 
 typedef struct pf_ctx pf_ctx;
 
@@ -167,7 +171,8 @@ int pf_ls(pf_ctx* ctx, const float* const* times, const float* const* mags,
  * derivative (0); out is [curve][k].  On such a grid the phases of one point
  * advance by the same angle from one frequency to the next, so besides the
  * MUFU sine / cosine per evaluation the autotuner can pick, per length
- * class, an angle-addition recurrence along the grid (PF_TRIG_* forces one).
+ * class, an angle-addition recurrence along the grid or a non-uniform FFT
+ * (PF_TRIG_* forces one).
  * Chosen form only (PF_MODE_CHOSEN; PF_FOLD_EXACT for an FP64 phase);
  * CUDA arithmetic only (PF_SEM_CPU is PF_EUNSUPPORTED).  Magnitudes as
  * pf_ls.  The device-pointer variant takes CSR curves as pf_ls_dev. */

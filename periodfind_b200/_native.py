@@ -40,6 +40,7 @@ PF_BINS_SHARED = 0x40000
 PF_ONE_LAUNCH = 0x80000
 PF_HOST_NORMALIZE = 0x100000
 PF_HOST_CENTER = 0x200000
+PF_TRIG_TRANSFORM = 0x400000
 PF_PREP_CENTER, PF_PREP_NORMALIZE = 1, 2
 PF_ALGO_CE, PF_ALGO_AOV, PF_ALGO_LS = 0, 1, 2
 

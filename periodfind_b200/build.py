@@ -41,6 +41,7 @@ UNITS = {
     "pf_api.cu": ["-Xcompiler", "-ffp-contract=off"],  # host float32 arithmetic as numpy
     "pf_noalloc.cu": [],
     "pf_lsgrad.cu": [],
+    "pf_nufft.cu": ["-use_fast_math"],
     "pf_stats.cu": ["-fmad=false"],  # numpy's float32 arithmetic, one rounding per operation
 }
 

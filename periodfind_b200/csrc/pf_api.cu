@@ -171,6 +171,8 @@ struct pf_ctx {
     bool staged_pending = false, done_recorded = false, timed_pending = false;
     std::string err;
     DevBuf d_in, d_aux32, d_aux64, d_out, d_pidx, d_pval, d_pack, d_misc, d_stamps, d_stat;
+    DevBuf d_nufft;  // the non-uniform FFT's table (constants)
+    bool nufft_ready = false;
     DevBuf d_bins;  // pf_bin_counts: raw bin counts per cell
     // pf_prepare_mags_dev: the curve offsets on the device, and the event
     // after the last kernel that read them (the buffer is rewritten only
@@ -850,6 +852,10 @@ uint64_t queue_items(const Job& j, uint64_t n_curves, int per_item) {
     return n_curves * j.n_pdt * ((j.n_per + per_item - 1) / per_item);
 }
 
+// The non-uniform FFT is a candidate from this many frequencies on (a block
+// costs the same however few of its kNufftModes are asked for).
+constexpr uint64_t kNufftMinFreqs = 1024;
+
 std::string tune_key(const Job& j, const FoldConfig& c, int cls) {
     char b[160];
     snprintf(b, sizeof(b), "%s %s%s%s%s ph=%u mag=%u pdt=%s sem=%s class=%s",
@@ -857,7 +863,8 @@ std::string tune_key(const Job& j, const FoldConfig& c, int cls) {
              c.kind == KIND_BIN ? "bin" : (c.fold == FOLD_DF ? "fold-split" : "fold-exact"),
              c.cnt16 ? "-cnt16" : "", c.ref_stats ? "-refstats" : "",
              j.fgrid ? ((j.mode & PF_TRIG_SINCOS) ? "-fgrid-sincos"
-                        : (j.mode & PF_TRIG_RECURRENCE) ? "-fgrid-recurrence" : "-fgrid")
+                        : (j.mode & PF_TRIG_RECURRENCE) ? "-fgrid-recurrence"
+                        : j.n_per < kNufftMinFreqs ? "-fgrid-short" : "-fgrid")
                      : (j.mode & PF_BINS_SHARED) ? "-shared-bins" : "",
              j.n_phase, c.algo == ALGO_CE ? j.n_mag : 0u, j.n_pdt > 1 ? "many" : "one",
              use_cpu_semantics(j.mode) ? "cpu" : "cuda", class_name(cls));
@@ -866,6 +873,12 @@ std::string tune_key(const Job& j, const FoldConfig& c, int cls) {
 
 cudaError_t launch_fold_sem(const Job& j, const FoldConfig& c, const FoldParams& p,
                             uint32_t n_work, cudaStream_t s) {
+    if (c.kind == KIND_NUFFT) {
+        const uint32_t blocks = (p.n_per + kNufftModes - 1) / kNufftModes;
+        const NufftParams q{p.t,    p.m,  p.curves, p.q.order, p.nufft_deconv, p.n_per,
+                            blocks, p.f0, p.df,     p.out,     p.stamps};
+        return launch_nufft(q, n_work / blocks, s);
+    }
     return use_cpu_semantics(j.mode) ? launch_fold_cpusem(c, p, n_work, s)
                                      : launch_fold_cudasem(c, p, n_work, s);
 }
@@ -885,11 +898,12 @@ int tuned_config(pf_ctx* ctx, const Job& j, const FoldConfig& base, int cls, uin
                  FoldConfig& out) {
     out = base;
     // LS on a uniform frequency grid: the trig form is a candidate axis too
-    // (MUFU sin / cos per evaluation, or the recurrence along the grid with
-    // 4 or 8 frequencies per thread); PF_TRIG_* keeps one form.
+    // (MUFU sin / cos per evaluation, the recurrence along the grid with 4 or
+    // 8 frequencies per thread, or the non-uniform FFT); PF_TRIG_* keeps one.
     const bool rec_ok = j.fgrid && base.algo == ALGO_LS && base.fold == FOLD_DF;
     const bool only_rec = rec_ok && (j.mode & PF_TRIG_RECURRENCE);
-    const bool no_rec = !rec_ok || (j.mode & PF_TRIG_SINCOS);
+    const bool only_fft = rec_ok && !only_rec && (j.mode & PF_TRIG_TRANSFORM);
+    const bool no_rec = !rec_ok || only_fft || (j.mode & PF_TRIG_SINCOS);
     // PF_BINS_SHARED takes the shared-histogram binning where the curves fit
     // it.  It is no candidate otherwise: its samples were 1.3-5x the
     // privatised form's on every class measured, before that form's newer
@@ -901,6 +915,11 @@ int tuned_config(pf_ctx* ctx, const Job& j, const FoldConfig& base, int cls, uin
         out.block = 256;
         out.rounds = 8;
         out.persist = false;
+    }
+    if (only_fft) {
+        out.kind = KIND_NUFFT;
+        out.persist = false;
+        return PF_OK;
     }
     if (only_warp) {
         out.kind = KIND_BINWARP;
@@ -985,6 +1004,13 @@ int tuned_config(pf_ctx* ctx, const Job& j, const FoldConfig& base, int cls, uin
                     t.persist = persist != 0;
                     cands.push_back(t);
                 }
+    }
+    if (rec_ok && !only_rec && !no_rec && j.n_per >= kNufftMinFreqs) {
+        FoldConfig t = base;
+        t.kind = KIND_NUFFT;
+        t.rounds = 1;
+        t.persist = false;
+        cands.push_back(t);
     }
     // Fastest of `reps` timed launches of candidate t on the sample.
     auto time_cand = [&](const FoldConfig& t, int reps, float& ms) -> int {
@@ -1235,6 +1261,17 @@ int device_pipeline(pf_ctx* ctx, const Job& j, const Layout& L, const FoldConfig
         }
         ctx->launches++;
     }
+    if (j.fgrid && !ctx->nufft_ready) {
+        if ((rc = ensure_dev(ctx, ctx->d_nufft, (kNufftModes / 2 + 1) * sizeof(float))) != PF_OK)
+            return rc;
+        PF_CUDA(launch_nufft_deconv((float*)ctx->d_nufft.p, s), "deconvolution table kernel");
+        ctx->launches++;
+        // A captured launch has not run yet.
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        PF_CUDA(cudaStreamIsCapturing(s, &cap), "capture query");
+        ctx->nufft_ready = cap == cudaStreamCaptureStatusNone;
+    }
+    p.nufft_deconv = (const float*)ctx->d_nufft.p;
     p.stamps = nullptr;
     Stage stage_fold(j.algo == ALGO_LS ? "pf LS fold" : j.algo == ALGO_CE ? "pf CE bins"
                                                                           : "pf AOV bins");
@@ -1894,7 +1931,7 @@ void pf_ctx_destroy(pf_ctx* ctx) {
     if (ctx->prep_pending) cudaEventSynchronize(ctx->ev_prep);
     for (DevBuf* b : {&ctx->d_in, &ctx->d_aux32, &ctx->d_aux64, &ctx->d_out, &ctx->d_pidx,
                       &ctx->d_pval, &ctx->d_pack, &ctx->d_misc, &ctx->d_stamps, &ctx->d_stat, &ctx->d_bins,
-                      &ctx->d_prep, &ctx->d_in2})
+                      &ctx->d_nufft, &ctx->d_prep, &ctx->d_in2})
         if (b->p) cudaFree(b->p);
     if (ctx->h_in.p) cudaFreeHost(ctx->h_in.p);
     if (ctx->h_res.p) cudaFreeHost(ctx->h_res.p);
@@ -1960,6 +1997,7 @@ int pf_tuning_report(const pf_ctx* ctx, char* buf, uint64_t len) {
                  "%s: %sblock=%d rounds=%d cells=%d %s sample_ms=%.3f slowest_ms=%.3f candidates=%u\n",
                  kv.first.c_str(),
                  kv.second.kind == KIND_LSREC ? "trig=recurrence "
+                 : kv.second.kind == KIND_NUFFT ? "trig=transform "
                  : kv.second.kind == KIND_BINWARP ? "bins=shared-atomic "
                  : kv.second.kind == KIND_BIN ? "bins=privatised "
                  : (kv.second.kind == KIND_FOLD && kv.first.find("fgrid") != std::string::npos)

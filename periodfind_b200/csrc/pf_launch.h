@@ -14,7 +14,10 @@ namespace pfk {
 // KIND_BINWARP: the chosen CE / AOV binning with one shared histogram per
 // warp and trial period, filled with shared atomics (pf_binwarp.cuh), the
 // alternative to KIND_BIN's per-thread privatised histograms.
-enum : int { KIND_FOLD = 0, KIND_BIN = 1, KIND_LSREC = 2, KIND_BINWARP = 3 };
+// KIND_NUFFT: Lomb-Scargle on a uniform frequency grid by a non-uniform FFT
+// (pf_nufft.cu); an item is kNufftModes frequencies.
+enum : int { KIND_FOLD = 0, KIND_BIN = 1, KIND_LSREC = 2, KIND_BINWARP = 3, KIND_NUFFT = 4 };
+constexpr int kNufftModes = 4096;
 constexpr uint32_t kWarpMaxPoints = 1024;  // KIND_BINWARP: longest curve it stages
 constexpr uint32_t kRecTileBytes = 512 * 16;  // lsrec_kernel's staged points
 
@@ -24,7 +27,7 @@ constexpr uint32_t kRecTileBytes = 512 * 16;  // lsrec_kernel's staged points
 // counter) or statically (one CTA per item).  The reference fold and the
 // all-FP32 study fold take one CTA per item of a host-built list.
 __host__ __device__ constexpr bool uses_queue(int kind, int fold) {
-    return kind == KIND_BIN || kind == KIND_LSREC || kind == KIND_BINWARP || fold == FOLD_EXACT ||
+    return kind == KIND_BIN || kind == KIND_LSREC || kind == KIND_BINWARP || kind == KIND_NUFFT || fold == FOLD_EXACT ||
            fold == FOLD_DF;
 }
 
@@ -49,6 +52,7 @@ size_t fold_smem(const FoldConfig& c, uint32_t n_phase, uint32_t n_mag);
 
 // Periods in one work item of a queue kernel.
 inline int item_periods(const FoldConfig& c) {
+    if (c.kind == KIND_NUFFT) return kNufftModes;
     int n = c.block;
     if ((c.kind == KIND_BIN || c.kind == KIND_LSREC) && c.rounds > 1) n *= c.rounds;
     if (c.kind == KIND_BIN && c.cells > 1) n *= c.cells;
@@ -120,6 +124,27 @@ cudaError_t launch_phase_probe_cudasem(int fold, const float* t, uint64_t n,
 cudaError_t launch_phase_probe_cpusem(int fold, const float* t, uint64_t n,
                                       const float* periods, uint64_t n_per, float period_dt,
                                       float* out, cudaStream_t s);
+
+// Lomb-Scargle on a uniform frequency grid by a non-uniform FFT (pf_nufft.cu):
+// a CTA per (curve of `order`, block of kNufftModes frequencies).
+struct NufftParams {
+    const float* t;
+    const float* m;
+    const CurveDesc* curves;
+    const uint32_t* order;
+    const float* deconv;  // launch_nufft_deconv's table
+    uint32_t n_freq;
+    uint32_t blocks;      // per curve
+    double f0, df;
+    float* out;           // [curve][n_freq]
+    unsigned long long* stamps;
+};
+// The normal matrix counts as near singular where its determinant is below
+// this fraction of n^2 (n^2 / 4 for well spread phases).
+constexpr float kNufftSingular = 1e-3f;
+cudaError_t launch_nufft(const NufftParams& p, uint32_t n_curves, cudaStream_t s);
+// The kernel transform's inverse, kNufftModes / 2 + 1 floats.
+cudaError_t launch_nufft_deconv(float* deconv, cudaStream_t s);
 
 // Preparation kernels (pf_prep.cu).
 // max |t| over n packed points into *tmax_bits (float bits; zeroed first).

@@ -1,0 +1,356 @@
+// pf_nufft.cu -- Lomb-Scargle sums on a uniform frequency grid by a
+// non-uniform FFT.
+//
+// On the grid f_k = f0 + k df the two sums the power needs,
+//     S_k = sum_i y_i e^{2 pi i t_i f_k},   Q_k = sum_i e^{4 pi i t_i f_k}
+// (mag_cos + i mag_sin, and cos_cos = (n + Re Q) / 2, cos_sin = Im Q / 2),
+// are Fourier sums over points at x_i = t_i df on the unit circle.  The
+// direct kernels (pf_lsrec.cuh, pf_fold.cuh) cost n operations per
+// frequency.  Here a CTA takes one curve and kNufftModes consecutive
+// frequencies around f_c: it spreads the points' values y_i e^{2 pi i t_i f_c}
+// onto a grid of twice as many cells with a kernel of width kW cells, takes
+// one FFT of the grid in shared memory, and divides each mode by the kernel's
+// transform (Dutt and Rokhlin 1993; the kernel exp(beta (sqrt(1 - z^2) - 1))
+// and beta = 2.3 kW are those of Barnett, Magland and af Klinteberg 2019,
+// whose error at width 8 is about 1e-7 of the norm of the input).  Cost per
+// block: two FFTs of 8192 points and about kW grid updates per point,
+// whatever the number of frequencies a point is needed at.
+//
+// Arithmetic: phases and grid positions are reduced in FP64 (the centre
+// phase t f_c and t df are good to 1e-11 turns), values, kernel and FFT are
+// FP32.  The spreading is exact in any order, so results are the same from run
+// to run: a tile of at most 512 points is added to the grid with 32-bit integer
+// reductions in units of 2^-31 of 512 times the largest value (2^-23 of one
+// rounding), and then taken into FP32 registers, a thread holding the 16 cells
+// that its first FFT pass needs.  (Float sums kept in order by giving each
+// cell to one warp were 2.5 times slower on long curves: 1.52 against 0.59 ms
+// for 83 curves of 4096-16384 points x 50000 frequencies.)
+//
+// Measured, 300 curves of 64-16384 points x 50000 frequencies: 14.95 ms with
+// the recurrence, 1.02 ms with this form; error of the power against FP64
+// 6.1e-6 and 5.0e-7 (2-norm).  Bound: short curves by the FFTs (about 29000 SM
+// cycles a block: barriers and shared memory), long ones by the spreading's
+// issue slots (staging arithmetic, 16 reductions per point and sum).  The
+// direct sums stay for grids below kNufftMinFreqs and where they are faster
+// on the tuner's sample.
+//
+// Cells where the normal matrix is near singular (f = 0, or a grid frequency
+// on which the sampling aliases) amplify any error of the sums, and the
+// direct sums there can be exactly singular: those cells are evaluated again
+// point by point, a warp per cell.
+#define PF_SEM_CPU_TU 0
+#define PF_KNS sem_cuda_nufft
+#include "pf_fold.cuh"
+
+namespace pfk {
+namespace PF_KNS {
+
+constexpr int kM = 8192;                 // grid cells (transform length)
+constexpr int kThreads = kM / 16;        // 16 grid cells per thread and pass
+constexpr int kW = 8;                    // kernel width in cells
+constexpr float kBeta = 2.3f * kW;
+constexpr int kTilePts = kThreads;       // points added between two flushes, one per thread
+static_assert(kNufftModes == kM / 2, "two grid cells per mode");
+
+// Grid storage: one float skipped every 16, so that the strided stores of
+// the first pass fall on different banks.
+__device__ __forceinline__ int pad(int i) { return i + (i >> 4); }
+constexpr int kPadded = kM + kM / 16;
+
+struct Smem {
+    float re[kPadded], im[kPadded];  // while spreading: integers
+};
+
+__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
+    return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) {
+    return make_float2(a.x + b.x, a.y + b.y);
+}
+__device__ __forceinline__ float2 csub(float2 a, float2 b) {
+    return make_float2(a.x - b.x, a.y - b.y);
+}
+// Four-point transform with positive exponent, in place.
+__device__ __forceinline__ void fft4(float2& x0, float2& x1, float2& x2, float2& x3) {
+    const float2 a = cadd(x0, x2), b = csub(x0, x2), c = cadd(x1, x3), e = csub(x1, x3);
+    const float2 d = make_float2(-e.y, e.x);
+    x0 = cadd(a, c);
+    x1 = cadd(b, d);
+    x2 = csub(a, c);
+    x3 = csub(b, d);
+}
+// Sixteen-point transform with positive exponent: X[k] ends in v[k].
+__device__ __forceinline__ void fft16(float2 (&v)[16]) {
+    constexpr float c1 = 0.92387953251128674f, s1 = 0.38268343236508977f;
+    constexpr float h = 0.70710678118654752f;
+#pragma unroll
+    for (int n2 = 0; n2 < 4; n2++) fft4(v[n2], v[4 + n2], v[8 + n2], v[12 + n2]);
+    // v[4 k1 + n2] times e^{2 pi i n2 k1 / 16}
+    v[5] = cmul(v[5], make_float2(c1, s1));
+    v[6] = cmul(v[6], make_float2(h, h));
+    v[7] = cmul(v[7], make_float2(s1, c1));
+    v[9] = cmul(v[9], make_float2(h, h));
+    v[10] = make_float2(-v[10].y, v[10].x);
+    v[11] = cmul(v[11], make_float2(-h, h));
+    v[13] = cmul(v[13], make_float2(s1, c1));
+    v[14] = cmul(v[14], make_float2(-h, h));
+    v[15] = cmul(v[15], make_float2(-c1, -s1));
+#pragma unroll
+    for (int k1 = 0; k1 < 4; k1++) fft4(v[4 * k1], v[4 * k1 + 1], v[4 * k1 + 2], v[4 * k1 + 3]);
+    // X[k1 + 4 k2] is in v[4 k1 + k2]: transpose.
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+        for (int b = a + 1; b < 4; b++) {
+            const float2 t = v[4 * a + b];
+            v[4 * a + b] = v[4 * b + a];
+            v[4 * b + a] = t;
+        }
+}
+
+// One radix-16 pass of the self-sorting FFT over the grid: sub-transforms of
+// length NS become ones of length 16 NS.  The first (NS = 1) takes its input
+// in v, the others from the grid.
+template <int NS>
+__device__ __forceinline__ void pass16(Smem& sm, float2 (&v)[16]) {
+    const int tid = threadIdx.x;
+    const int q = tid % NS;
+    if constexpr (NS > 1) {
+#pragma unroll
+        for (int r = 0; r < 16; r++) {
+            const int i = pad(tid + r * kThreads);
+            v[r] = make_float2(sm.re[i], sm.im[i]);
+        }
+        float2 w[16];
+        sincospif(2.0f * (float)q / (float)(16 * NS), &w[1].y, &w[1].x);
+        v[1] = cmul(v[1], w[1]);
+#pragma unroll
+        for (int r = 2; r < 16; r++) {
+            w[r] = (r & 1) ? cmul(w[r - 1], w[1]) : cmul(w[r / 2], w[r / 2]);
+            v[r] = cmul(v[r], w[r]);
+        }
+    }
+    fft16(v);
+    __syncthreads();
+    const int o = (tid / NS) * (NS * 16) + q;
+#pragma unroll
+    for (int r = 0; r < 16; r++) {
+        const int i = pad(o + r * NS);
+        sm.re[i] = v[r].x;
+        sm.im[i] = v[r].y;
+    }
+    __syncthreads();
+}
+
+// Spread one of the two sums' points and transform the grid.  After it, the
+// three radix-16 passes are done and mode(j) below finishes the last, radix-2
+// one.  MULT = 1: S (values y); MULT = 2: Q (values 1).  `scale` turns
+// a value into grid units.
+template <int MULT>
+__device__ __forceinline__ void spread_and_transform(Smem& sm, const float* __restrict__ t,
+                                                     const float* __restrict__ y, uint32_t n,
+                                                     double fc, double df, float scale) {
+    const int tid = threadIdx.x;
+    int* gre = reinterpret_cast<int*>(sm.re);
+    int* gim = reinterpret_cast<int*>(sm.im);
+    float2 v[16];
+#pragma unroll
+    for (int r = 0; r < 16; r++) {
+        const int i = pad(tid + r * kThreads);
+        gre[i] = 0;
+        gim[i] = 0;
+        v[r] = make_float2(0.0f, 0.0f);
+    }
+    __syncthreads();
+    // Times come sorted, so neighbouring points land in neighbouring cells: a
+    // tile takes every tiles-th point of the curve, which keeps the lanes of
+    // a warp apart on the grid.
+    const uint32_t tiles = (n + kTilePts - 1) / kTilePts;
+    for (uint32_t k = 0; k < tiles; k++) {
+        const uint64_t at = (uint64_t)tid * tiles + k;
+        if (at < n) {
+            const double td = (double)t[at];
+            double th = td * (fc * MULT);
+            th -= rint(th);
+            float s, c;
+            sincospif(2.0f * (float)th, &s, &c);
+            const float a = MULT == 1 ? scale * y[at] : scale;
+            s *= a;
+            c *= a;
+            double x = td * (df * MULT);
+            x -= floor(x);
+            const double u = x * (double)kM;
+            const double m = floor(u);
+            const float fr = (float)(u - m);
+            const int first = (int)m - (kW / 2 - 1);
+#pragma unroll
+            for (int l = 0; l < kW; l++) {
+                const float z = ((float)(l - (kW / 2 - 1)) - fr) * (2.0f / kW);
+                const float r = sqrtf(fmaxf(1.0f - z * z, 0.0f));
+                const float w = __expf(kBeta * (r - 1.0f));
+                const int i = pad((first + l) & (kM - 1));
+                atomicAdd(&gre[i], __float2int_rn(c * w));
+                atomicAdd(&gim[i], __float2int_rn(s * w));
+            }
+        }
+        __syncthreads();
+        const bool more = k + 1 < tiles;
+#pragma unroll
+        for (int r = 0; r < 16; r++) {
+            const int i = pad(tid + r * kThreads);
+            v[r].x += (float)gre[i];
+            v[r].y += (float)gim[i];
+            if (more) {
+                gre[i] = 0;
+                gim[i] = 0;
+            }
+        }
+        __syncthreads();
+    }
+    pass16<1>(sm, v);
+    pass16<16>(sm, v);
+    pass16<256>(sm, v);
+}
+
+// Mode of index j (0 <= j < kM / 2) after the radix-16 passes: kappa = j for
+// j < kM / 4, else j - kM / 2 (the last pass gives two modes per j, of which
+// exactly one lies in the kept half).
+__device__ __forceinline__ float2 mode(const Smem& sm, int j) {
+    const int a = pad(j), b = pad(j + kM / 2);
+    float2 w;
+    sincospif(2.0f * (float)j / (float)kM, &w.y, &w.x);
+    const float2 x = make_float2(sm.re[a], sm.im[a]);
+    const float2 z = cmul(make_float2(sm.re[b], sm.im[b]), w);
+    return j < kM / 4 ? cadd(x, z) : csub(x, z);
+}
+
+__global__ void __launch_bounds__(kThreads, 2)
+    nufft_kernel(const NufftParams p) {
+    extern __shared__ __align__(16) unsigned char nsm[];
+    Smem& sm = *reinterpret_cast<Smem*>(nsm);
+    const uint32_t c = p.order[blockIdx.x / p.blocks];
+    const uint32_t k0 = (blockIdx.x % p.blocks) * (uint32_t)kNufftModes;
+    const CurveDesc cd = p.curves[c];
+    const float* t = p.t + cd.off;
+    const float* y = p.m + cd.off;
+    const uint32_t n = cd.n;
+    if (p.stamps && threadIdx.x == 0) p.stamps[2 * (size_t)blockIdx.x] = global_ns();
+    const double fc = p.f0 + (double)(k0 + kNufftModes / 2) * p.df;
+    constexpr int kPer = kNufftModes / kThreads;  // modes per thread
+
+    // Largest |y|; a point that is not finite makes every value NaN, as in
+    // the direct sums.
+    __shared__ unsigned s_max;
+    if (threadIdx.x == 0) s_max = 0u;
+    __syncthreads();
+    unsigned my_max = 0u;
+    bool bad = false;
+    for (uint32_t i = threadIdx.x; i < n; i += kThreads) {
+        const float yi = y[i];
+        bad = bad || !(fabsf(yi) < INFINITY) || !(fabsf(t[i]) < INFINITY);
+        my_max = max(my_max, __float_as_uint(fabsf(yi)));
+    }
+    my_max = __reduce_max_sync(0xffffffffu, my_max);
+    if ((threadIdx.x & 31) == 0) atomicMax(&s_max, my_max);
+    bad = __syncthreads_or(bad ? 1 : 0) != 0;
+    const float y_max = __uint_as_float(s_max);
+    constexpr float kFull = 2147483392.0f / kTilePts;  // below 2^31 / kTilePts
+    // (squares below 1e-60 are zero in the direct sums too)
+    const float y_scale = y_max > 1e-30f ? kFull / y_max : 0.0f;
+    const float nan = __uint_as_float(0x7FC00000u);
+    const float y_unit = bad ? nan : y_max * (1.0f / kFull), q_unit = bad ? nan : 1.0f / kFull;
+
+    float2 q[kPer];
+    spread_and_transform<2>(sm, t, y, n, fc, p.df, kFull);
+#pragma unroll
+    for (int i = 0; i < kPer; i++) q[i] = mode(sm, threadIdx.x + i * kThreads);
+    __syncthreads();
+    spread_and_transform<1>(sm, t, y, n, fc, p.df, y_scale);
+
+    float* out = p.out + (size_t)c * p.n_freq;
+    unsigned again = 0;  // the thread's near-singular modes
+#pragma unroll
+    for (int i = 0; i < kPer; i++) {
+        const int j = threadIdx.x + i * kThreads;
+        const int kappa = j < kM / 4 ? j : j - kM / 2;
+        const uint64_t k = (uint64_t)k0 + (uint32_t)(kappa + kNufftModes / 2);
+        if (k >= p.n_freq) continue;
+        const float dc = p.deconv[kappa < 0 ? -kappa : kappa];
+        const float2 sv = mode(sm, j);
+        const float dy = dc * y_unit, dq = dc * q_unit;
+        const LSAcc a{sv.x * dy, sv.y * dy, 0.5f * fmaf(q[i].x, dq, (float)n),
+                      0.5f * q[i].y * dq};
+        const float det = a.cos_cos * ((float)n - a.cos_cos) - a.cos_sin * a.cos_sin;
+        if (!(det > kNufftSingular * (float)n * (float)n)) again |= 1u << i;
+        out[k] = ls_power(a, n);
+    }
+    // Near-singular modes point by point, a warp each.
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (int i = 0; i < kPer; i++) {
+        unsigned todo = __ballot_sync(0xffffffffu, (again >> i) & 1u);
+        while (todo) {
+            const int src = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const int j = (int)(threadIdx.x & ~31u) + src + i * kThreads;
+            const int kappa = j < kM / 4 ? j : j - kM / 2;
+            const uint32_t k = k0 + (uint32_t)(kappa + kNufftModes / 2);
+            const double f = p.f0 + (double)k * p.df;
+            LSAcc a{0.0f, 0.0f, 0.0f, 0.0f};
+            for (uint32_t e = lane; e < n; e += 32) {
+                double th = (double)t[e] * f;
+                th -= rint(th);
+                float s, co;
+                sincosf(kTwoPi * (float)th, &s, &co);
+                const float ye = y[e];
+                a.mag_cos += ye * co;
+                a.mag_sin += ye * s;
+                a.cos_cos += co * co;
+                a.cos_sin += co * s;
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                a.mag_cos += __shfl_xor_sync(0xffffffffu, a.mag_cos, o);
+                a.mag_sin += __shfl_xor_sync(0xffffffffu, a.mag_sin, o);
+                a.cos_cos += __shfl_xor_sync(0xffffffffu, a.cos_cos, o);
+                a.cos_sin += __shfl_xor_sync(0xffffffffu, a.cos_sin, o);
+            }
+            if (lane == 0) out[k] = ls_power(a, n);
+        }
+    }
+    if (p.stamps && threadIdx.x == 0) p.stamps[2 * (size_t)blockIdx.x + 1] = global_ns();
+}
+
+// 1 / (the kernel's transform at mode k), k = 0 .. kNufftModes / 2: the
+// trapezoidal rule on the even kernel, which has all but vanished at its ends.
+__global__ void nufft_deconv_kernel(float* __restrict__ deconv) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k > kNufftModes / 2) return;
+    constexpr int kNodes = 96;
+    double sum = 0.5;  // half the value at z = 0
+    for (int i = 1; i < kNodes; i++) {
+        const double z = (double)i / kNodes;
+        sum += exp((double)kBeta * (sqrt(1.0 - z * z) - 1.0)) *
+               cospi((double)k * kW * z / (double)kM);
+    }
+    deconv[k] = (float)(1.0 / (sum * kW / kNodes));
+}
+
+}  // namespace PF_KNS
+
+cudaError_t launch_nufft_deconv(float* deconv, cudaStream_t s) {
+    PF_KNS::nufft_deconv_kernel<<<(kNufftModes / 2 + 64) / 64, 64, 0, s>>>(deconv);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_nufft(const NufftParams& p, uint32_t n_curves, cudaStream_t s) {
+    if (n_curves == 0) return cudaSuccess;
+    const int smem = (int)sizeof(PF_KNS::Smem);
+    cudaError_t e = cudaFuncSetAttribute(PF_KNS::nufft_kernel,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    PF_KNS::nufft_kernel<<<n_curves * p.blocks, PF_KNS::kThreads, smem, s>>>(p);
+    return cudaGetLastError();
+}
+
+}  // namespace pfk
