@@ -2375,12 +2375,13 @@ int pf_prepare_mags_dev(pf_ctx* ctx, const float* d_mags, const int64_t* offsets
     if (!offsets) return fail(ctx, PF_EINVAL, "offsets is NULL");
     if (n_curves > 0x7FFFFFFFull) return fail(ctx, PF_EINVAL, "too many curves");
     if (offsets[0] < 0) return fail(ctx, PF_EINVAL, "offsets[0] is negative");
-    uint32_t leaf_cap = 1;
+    uint32_t leaf_cap = 1, max_len = 0;
     for (uint64_t c = 0; c < n_curves; c++) {
         const int64_t len = offsets[c + 1] - offsets[c];
         if (len < 0 || len > 0xFFFFFFFFll)
             return fail(ctx, PF_EINVAL, "offsets must be non-decreasing (curve %llu)",
                         (unsigned long long)c);
+        max_len = std::max(max_len, (uint32_t)len);
         if (kind == PF_PREP_CENTER && len > 0)
             leaf_cap = std::max(leaf_cap, stats_leaf_count((uint32_t)len));
     }
@@ -2399,7 +2400,7 @@ int pf_prepare_mags_dev(pf_ctx* ctx, const float* d_mags, const int64_t* offsets
     PF_CUDA(cudaMemcpyAsync(ctx->d_prep.p, offsets, (n_curves + 1) * 8, cudaMemcpyHostToDevice,
                             s),
             "H2D offsets");
-    PF_CUDA(launch_prep_mags(d_mags, (const int64_t*)ctx->d_prep.p, n_curves, leaf_cap, kind,
+    PF_CUDA(launch_prep_mags(d_mags, (const int64_t*)ctx->d_prep.p, n_curves, max_len, kind,
                              d_out, s),
             "magnitude preparation launch");
     PF_CUDA(cudaEventRecord(ctx->ev_prep, s), "event");
