@@ -1815,6 +1815,9 @@ int run_fpw(pf_ctx* ctx, const float* const* times, const float* const* mags,
     p.out = (float*)ctx->d_out.p;
     p.tmax = tmax;
     p.edge_d = edge_guard(n_bins);
+    const uint32_t edge32 = (p.edge_d << 12) / n_bins + 2u;  // D (see device_pipeline)
+    p.magic32 = 6755399441055744.0 + (double)edge32;
+    p.edge32_lim = 2u * edge32 * n_bins;
     const bool exact = (mode & PF_MODE_CHOSEN) != 0;
     PF_CUDA(cudaEventRecord(ctx->ev0, s), "event");
     PF_CUDA((mode & PF_SEM_CPU) ? launch_fpw_cpusem(p, exact, n_curves, s)

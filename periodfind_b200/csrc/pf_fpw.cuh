@@ -7,10 +7,9 @@
 // value is sum over bins with V > 0 of Y^2 / (2 V).  Maximum is best.
 //
 // Decomposition: a CTA per (curve, period derivative, tile of BLOCK trial
-// periods); thread j owns one period for the whole curve and keeps its own
+// periods); thread j owns one period (the chosen form: two) for the whole curve and keeps its own
 // V and Y in shared memory ([bin][thread], so a warp's updates touch
-// consecutive words: the chosen form as (V, Y) float2 pairs, one 8-byte
-// access per update; the plain form as V rows then Y rows), adding the
+// consecutive words), adding the
 // points in curve order -- the Rust path's order, so the sums round as it
 // does.  The curve streams through shared memory in 16-byte point records,
 // 256 points per tile.
@@ -22,12 +21,8 @@
 // with folded = (float)|q - floor(q)| for the correctly rounded quotient q.
 //
 // Plain form: that sequence for every point (FP64 divide).  Chosen form: the
-// bin from q' = t * RN(1/P) with a round-down floor and one round-down FMA
-// that yields floor(q' n_bins) and 20 fraction bits (the chosen CE / AOV bin
-// kernel's construction); a point whose fraction lies within the proven
-// guard of a bin edge takes the reference sequence instead (divide-free, the
-// same quotient).  Unlike the integer CE / AOV counters, float sums cannot
-// take a point back, so each point is tested before it is added.
+// CE / AOV bin kernel's fast bin, the reference sequence within the proven
+// guard of a bin edge (divide-free, the same quotient).
 #pragma once
 
 #ifndef PF_KNS
@@ -55,38 +50,102 @@ __device__ __forceinline__ uint32_t fpw_ref_bin(float folded, const FpwParams& p
 // the value is the best s^2 / (r (W - r)) over the windows of nb_min ..
 // nb_max consecutive bins (wrapping) whose weight fraction r / W lies in
 // (0, 1); 0 when W <= 0.
-template <int BLOCK, bool CHOSEN, bool BLS, int GROUP>
+//
+// FPW value of one cell from its bins (row k: ld(k) = (V, Y)).
+template <class LD>
+__device__ __forceinline__ float fpw_value(LD&& ld, uint32_t nb) {
+    float acc = 0.0f;
+    for (uint32_t k = 0; k < nb; k++) {
+        const float2 x = ld(k);
+        if (x.x > 0.0f) acc += x.y * x.y / (2.0f * x.x);
+    }
+    return acc;
+}
+
+// BLS values of CELLS cells at once (row k of cell c: ld(k, c), put(k, c, x)).
+// Prefix sums in place, in the reference's order (bls.rs:83-89): row k + 1
+// becomes row k + row k + 1.  Then every (phase, width) window, phase-major:
+// the window's start row is read once per phase.  The sums are the
+// reference's: end <= nb gives row[end] - row[phi] (x - y is x + (-y)
+// exactly), a wrapping window (total - row[phi]) + row[end - nb]; the maximum
+// does not depend on the order of the windows.
+template <int CELLS, class LD, class PUT>
+__device__ __forceinline__ void bls_values(LD&& ld, PUT&& put, uint32_t nb, uint32_t nb_min,
+                                           uint32_t nb_max, float (&acc)[CELLS]) {
+    float2 tot[CELLS];
+#pragma unroll
+    for (int c = 0; c < CELLS; c++) {
+        tot[c] = ld(0, c);
+        acc[c] = 0.0f;
+    }
+    for (uint32_t k = 0; k < nb; k++)
+#pragma unroll
+        for (int c = 0; c < CELLS; c++) {
+            float2 x = ld(k + 1, c);
+            x.x = tot[c].x + x.x;
+            x.y = tot[c].y + x.y;
+            put(k + 1, c, x);
+            tot[c] = x;
+        }
+    for (uint32_t phi = 0; phi < nb; phi++) {
+        float2 a[CELLS], rest[CELLS];
+#pragma unroll
+        for (int c = 0; c < CELLS; c++) {
+            a[c] = ld(phi, c);
+            rest[c] = make_float2(tot[c].x - a[c].x, tot[c].y - a[c].y);
+        }
+        // The windows that end in rows lo .. hi (consecutive), their sums
+        // row + base.  No branch in the loop, so that the loads and divides of
+        // several windows overlap (a cell outside the weight range scores 0,
+        // and a NaN score leaves the maximum as a comparison would).
+        auto windows = [&](uint32_t lo, uint32_t hi, const float2 (&base)[CELLS]) {
+#pragma unroll 4
+            for (uint32_t k = lo; k <= hi; k++) {
+#pragma unroll
+                for (int c = 0; c < CELLS; c++) {
+                    const float2 e = ld(k, c);
+                    const float r = e.x + base[c].x, sy = e.y + base[c].y;
+                    const float r_frac = r / tot[c].x;
+                    const float bls = (sy * sy) / (r * (tot[c].x - r));
+                    acc[c] = fmaxf(acc[c], r_frac > 0.0f && r_frac < 1.0f ? bls : 0.0f);
+                }
+            }
+        };
+        float2 minus[CELLS];
+#pragma unroll
+        for (int c = 0; c < CELLS; c++) minus[c] = make_float2(-a[c].x, -a[c].y);
+        windows(phi + nb_min, min(phi + nb_max, nb), minus);
+        // Wrapping: widths of at least nb - phi + 1.
+        if (phi + nb_max > nb)
+            windows(max(phi + nb_min, nb + 1u) - nb, phi + nb_max - nb, rest);
+    }
+    // No weight, no window.
+#pragma unroll
+    for (int c = 0; c < CELLS; c++)
+        if (!(tot[c].x > 0.0f)) acc[c] = 0.0f;
+}
+
+// The plain form.
+template <int BLOCK, bool BLS>
 __global__ void __launch_bounds__(BLOCK)
     fpw_kernel(const FpwParams p, uint32_t tiles_per_row) {
-    using TT = typename std::conditional<CHOSEN, double, float>::type;
     // One 16-byte record per staged point: a single 128-bit shared load.
     struct alignas(16) Point {
-        TT t;
-        float iv, ivy;
+        float t, iv, ivy;
     };
     constexpr uint32_t kRow0 = BLS ? 1u : 0u;  // rows before bin 0
     extern __shared__ __align__(16) unsigned char fsm[];
     Point* st = reinterpret_cast<Point*>(fsm);
-    // Per-thread bins, row k (bin k - kRow0) of thread tid: the chosen form
-    // keeps (V, Y) pairs, [row][BLOCK] float2, so a bin update is one 8-byte
-    // load and store; the plain form keeps V rows then Y rows.
+    // Per-thread bins: V rows then Y rows, row k (bin k - kRow0) of thread tid.
     float* bins = reinterpret_cast<float*>(st + kFpwTile);
     const uint32_t rows = p.n_bins + kRow0;
     auto ld = [&](uint32_t k) -> float2 {
-        if constexpr (CHOSEN)
-            return reinterpret_cast<const float2*>(bins)[k * BLOCK + threadIdx.x];
-        else
-            return make_float2(bins[k * BLOCK + threadIdx.x], bins[(rows + k) * BLOCK + threadIdx.x]);
+        return make_float2(bins[k * BLOCK + threadIdx.x], bins[(rows + k) * BLOCK + threadIdx.x]);
     };
     auto put = [&](uint32_t k, float2 x) {
-        if constexpr (CHOSEN) {
-            reinterpret_cast<float2*>(bins)[k * BLOCK + threadIdx.x] = x;
-        } else {
-            bins[k * BLOCK + threadIdx.x] = x.x;
-            bins[(rows + k) * BLOCK + threadIdx.x] = x.y;
-        }
+        bins[k * BLOCK + threadIdx.x] = x.x;
+        bins[(rows + k) * BLOCK + threadIdx.x] = x.y;
     };
-    __shared__ double warp_min[BLOCK / 32];
 
     const uint64_t cta = blockIdx.x;
     const uint32_t tile = (uint32_t)(cta % tiles_per_row);
@@ -101,160 +160,227 @@ __global__ void __launch_bounds__(BLOCK)
     const uint32_t n = p.len[c];
     const uint32_t nb = p.n_bins;
     for (uint32_t k = 0; k < rows; k++) put(k, make_float2(0.0f, 0.0f));
-    const float period = p.periods[active ? pi : (uint64_t)tile * BLOCK];
-    const float period_dt = p.pdts[d];
     Cell s;
-    cell_setup<CHOSEN ? FOLD_EXACT : FOLD_REF>(s, period, period_dt);
-    const bool has_pdt = period_dt != 0.0f;
-
-    // Chosen form: the fast bin is exact away from bin edges while
-    // |q| * n_bins < 2^30 (the same bound as the chosen CE / AOV kernels),
-    // checked for the CTA from max|t| and its smallest |P|.
-    bool fast = false, fast32 = false;
-    if constexpr (CHOSEN) {
-        double mn = fabs((double)period);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-        if ((tid & 31) == 0) warp_min[tid >> 5] = mn;
-        __syncthreads();
-        double pmin = warp_min[0];
-#pragma unroll
-        for (int k = 1; k < BLOCK / 32; k++) pmin = fmin(pmin, warp_min[k]);
-        const double qb = p.tmax / pmin + fabs((double)period_dt) * p.tmax * p.tmax /
-                                              (2.0 * pmin * pmin);
-        fast = qb * (double)nb < 1073741824.0;  // 2^30
-        // |q| < 2^19 as well: the one-FMA bin below.
-        fast32 = fast && qb < 524288.0;
-    }
-    const double nd20 = (double)nb * 1048576.0;
-    const uint32_t n_neg = 0u - nb;
-    const uint32_t edge_add = p.edge_d << 12;
-    const uint32_t edge_lim = (2u * p.edge_d) << 12;
-    // The guard in units of 2^-32 of a bin, widened by n_bins + 2 units for
-    // the truncation of the phase to 32 bits.
-    const uint32_t edge32_add = edge_add + nb + 2u;
-    const uint32_t edge32_lim = 2u * edge32_add;
-    const double y32 = s.yhi * 4294967296.0;  // RN(1/P) * 2^32, exact
-
-    // The reference's bin of point time t (the fast bin when the CTA's
-    // bound allows, the reference sequence near an edge or otherwise).
-    auto bin_of = [&](TT t) -> uint32_t {
-        if constexpr (CHOSEN) {
-            const double td = t;
-            if (fast32) {
-                // One FMA on the exact product t * (RN(1/P) * 2^32) leaves
-                // floor(frac(q') * 2^32) in the low word f; the 64-bit
-                // product f * n_bins holds the bin (high word) and the
-                // position within it (low word, for the edge test).
-                const double a = has_pdt ? td - s.c * td * td : td;
-                const double y = __fma_rd(a, y32, kMagic15);
-                const uint32_t f = (uint32_t)__double2loint(y);
-                const unsigned long long fn = (unsigned long long)f * nb;
-                if ((uint32_t)fn + edge32_add >= edge32_lim) return (uint32_t)(fn >> 32);
-            } else if (fast) {
-                const double a = has_pdt ? td - s.c * td * td : td;
-                const double qh = __dmul_rn(a, s.yhi);
-                const double r = __dadd_rd(qh, kMagic15);
-                const double y = __fma_rd(qh, nd20, kMagic15);
-                const uint32_t ylo = (uint32_t)__double2loint(y);
-                const uint32_t yhi = (uint32_t)__double2hiint(y);
-                // floor(q' n_bins) - n_bins floor(q'), biased by 2^31 by the
-                // magic constant's top mantissa bit.
-                const uint32_t b = __funnelshift_r(ylo, yhi, 20) +
-                                   (uint32_t)__double2loint(r) * n_neg - 0x80000000u;
-                if (ylo * 4096u + edge_add >= edge_lim) return b;
-            }
-            return fpw_ref_bin(has_pdt ? fold_exact<true>(td, s) : fold_exact<false>(td, s), p);
-        } else {
-            return fpw_ref_bin(fold_ref(t, s), p);
-        }
-    };
+    cell_setup<FOLD_REF>(s, p.periods[active ? pi : (uint64_t)tile * BLOCK], p.pdts[d]);
 
     for (uint32_t base = 0; base < n; base += kFpwTile) {
         const uint32_t cnt = min(kFpwTile, n - base);
         __syncthreads();
         for (uint32_t i = tid; i < cnt; i += BLOCK)
-            st[i] = Point{(TT)p.t[off + base + i], p.iv[off + base + i], p.ivy[off + base + i]};
+            st[i] = Point{p.t[off + base + i], p.iv[off + base + i], p.ivy[off + base + i]};
         __syncthreads();
         if (!active) continue;
-        uint32_t i = 0;
-        if constexpr (GROUP > 1) {
-            // GROUP points are read and binned before the first of their
-            // read-modify-writes: the staged tile and the bins share one
-            // shared-memory array, so a point read cannot move above an
-            // earlier bin store, and one point at a time would chain the
-            // point read, the bin arithmetic and the bin update per point.
-            // The updates stay in point order (same bin, same rounding).
-            for (; i + GROUP <= cnt; i += GROUP) {
-                Point q[GROUP];
-                uint32_t b[GROUP];
-#pragma unroll
-                for (int k = 0; k < GROUP; k++) q[k] = st[i + k];
-#pragma unroll
-                for (int k = 0; k < GROUP; k++) b[k] = bin_of(q[k].t);
-#pragma unroll
-                for (int k = 0; k < GROUP; k++) {
-                    float2 x = ld(b[k] + kRow0);
-                    x.x += q[k].iv;
-                    x.y += q[k].ivy;
-                    put(b[k] + kRow0, x);
-                }
-            }
-        }
 #pragma unroll 4
-        for (; i < cnt; i++) {
+        for (uint32_t i = 0; i < cnt; i++) {
             const Point pt = st[i];
-            const uint32_t bin = bin_of(pt.t);
-            float2 x = ld(bin + kRow0);
+            const uint32_t bin = fpw_ref_bin(fold_ref(pt.t, s), p) + kRow0;
+            float2 x = ld(bin);
             x.x += pt.iv;
             x.y += pt.ivy;
-            put(bin + kRow0, x);
+            put(bin, x);
         }
     }
     if (!active) return;
-    float acc = 0.0f;
-    if constexpr (BLS) {
-        // Prefix sums in place, in the reference's order (bls.rs:83-89):
-        // row k + 1 becomes row k + row k + 1.
-        float2 prev = ld(0);
-        for (uint32_t k = 0; k < nb; k++) {
-            float2 x = ld(k + 1);
-            x.x = prev.x + x.x;
-            x.y = prev.y + x.y;
-            put(k + 1, x);
-            prev = x;
-        }
-        const float w_total = prev.x, y_total = prev.y;
-        if (w_total > 0.0f) {
-            // Every (phase, width) window, phase-major: the window's start
-            // row is read once per phase.  The sums are the reference's:
-            // end <= nb gives row[end] - row[phi] (x - y is x + (-y)
-            // exactly), a wrapping window (total - row[phi]) + row[end - nb];
-            // the maximum does not depend on the order of the windows.
-            for (uint32_t phi = 0; phi < nb; phi++) {
-                const float2 a = ld(phi);
-                const float w_rest = w_total - a.x, y_rest = y_total - a.y;
-                for (uint32_t nbw = p.nb_min; nbw <= p.nb_max; nbw++) {
-                    const uint32_t end = phi + nbw;
-                    const bool wrap = end > nb;
-                    const float2 e = ld(wrap ? end - nb : end);
-                    const float r = e.x + (wrap ? w_rest : -a.x);
-                    const float sy = e.y + (wrap ? y_rest : -a.y);
-                    const float r_frac = r / w_total;
-                    if (r_frac > 0.0f && r_frac < 1.0f) {
-                        const float bls = (sy * sy) / (r * (w_total - r));
-                        if (bls > acc) acc = bls;
-                    }
-                }
-            }
-        }
-    } else {
-        for (uint32_t k = 0; k < nb; k++) {
-            const float2 x = ld(k);
-            if (x.x > 0.0f) acc += x.y * x.y / (2.0f * x.x);
-        }
+    float acc[1];
+    if constexpr (BLS)
+        bls_values<1>([&](uint32_t k, int) { return ld(k); },
+                      [&](uint32_t k, int, float2 x) { put(k, x); }, nb, p.nb_min, p.nb_max, acc);
+    else
+        acc[0] = fpw_value(ld, nb);
+    p.out[(uint64_t)c * (p.n_per * p.n_pdt) + pi * p.n_pdt + d] = acc[0];
+}
+
+// The chosen form: the bin from the one-FMA construction of the CE / AOV
+// bin kernel (pf_bin.cuh, fast_bin32: the guard rides in the FMA's constant,
+// so a point's edge test is its product's low word against a limit), a
+// thread holding CELLS trial periods, whose updates share the staged
+// point's load (2 up to 32 bins; 1 beyond, where shared memory holds so few
+// cells that the warps are needed to hide latency: BLS(50) kernel 5.2 ms with
+// two, 2.8 with one).  Four points are read and binned before the first of their
+// read-modify-writes (the staged tile and the bins share one array, so a
+// point read cannot move above an earlier bin store); a group with a point
+// near an edge corrects that point's bin first, as float sums cannot be
+// taken back.  Updates stay in point order (same bin, same rounding).
+//
+// Bound: the shared-memory pipe, 96% busy for FPW (per evaluation half a
+// 128-bit broadcast load, an 8-byte load and an 8-byte store), 75% for BLS.
+// FPW(10) with uncertainties, 100 curves x 4096 points x 10000 periods x 2:
+// 4.81 ms, the call from host arrays 9.35 -> 6.70 ms; BLS(50), 150 x 1500 x
+// 10000, whose 1250 windows per cell cost as much as its points: the call 5.50
+// -> 3.86 ms (4.15 ms with one window loop and a select per wrap).
+template <int BLOCK, bool BLS, int CELLS>
+__global__ void __launch_bounds__(BLOCK)
+    fpw_chosen_kernel(const FpwParams p, uint32_t tiles_per_row) {
+    struct alignas(16) Point {
+        double t;
+        float iv, ivy;
+    };
+    constexpr uint32_t kCols = BLOCK * CELLS;
+    constexpr uint32_t kRow0 = BLS ? 1u : 0u;  // rows before bin 0
+    extern __shared__ __align__(16) unsigned char fsm[];
+    Point* st = reinterpret_cast<Point*>(fsm);
+    // (V, Y) of row k (bin k - kRow0) of cell c of thread tid: one 8-byte
+    // access per update, a warp's on consecutive words.
+    float2* bins = reinterpret_cast<float2*>(st + kFpwTile) + threadIdx.x;
+    auto ld = [&](uint32_t k, int c) -> float2 { return bins[k * kCols + c * BLOCK]; };
+    auto put = [&](uint32_t k, int c, float2 x) { bins[k * kCols + c * BLOCK] = x; };
+    __shared__ double warp_min[BLOCK / 32];
+
+    const uint64_t cta = blockIdx.x;
+    const uint32_t tile = (uint32_t)(cta % tiles_per_row);
+    const uint64_t row = cta / tiles_per_row;     // curve * n_pdt + pdt
+    const uint64_t cv = row / p.n_pdt;
+    const uint32_t dt = (uint32_t)(row % p.n_pdt);
+    const int tid = threadIdx.x;
+    const uint64_t p0 = (uint64_t)tile * kCols, pi0 = p0 + tid;
+    const bool active = pi0 < p.n_per;  // a thread with any live cell runs all
+
+    const int64_t off = p.off[cv];
+    const uint32_t n = p.len[cv];
+    const uint32_t nb = p.n_bins;
+    for (uint32_t k = 0; k < nb + kRow0; k++)
+#pragma unroll
+        for (int c = 0; c < CELLS; c++) put(k, c, make_float2(0.0f, 0.0f));
+    const float period_dt = p.pdts[dt];
+    Cell s[CELLS];
+    double mn = INFINITY;
+#pragma unroll
+    for (int c = 0; c < CELLS; c++) {
+        const uint64_t pi = pi0 + (uint64_t)c * BLOCK;
+        const float period = p.periods[pi < p.n_per ? pi : p0];
+        cell_setup<FOLD_EXACT>(s[c], period, period_dt);
+        mn = fmin(mn, fabs((double)period));
     }
-    p.out[(uint64_t)c * (p.n_per * p.n_pdt) + pi * p.n_pdt + d] = acc;
+
+    // The fast bin is exact away from bin edges while |q| * n_bins < 2^30 (the
+    // same bound as the chosen CE / AOV kernels), checked for the CTA from
+    // max|t| and its smallest |P|.
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+    if ((tid & 31) == 0) warp_min[tid >> 5] = mn;
+    __syncthreads();
+    double pmin = warp_min[0];
+#pragma unroll
+    for (int k = 1; k < BLOCK / 32; k++) pmin = fmin(pmin, warp_min[k]);
+    const double qb =
+        p.tmax / pmin + fabs((double)period_dt) * p.tmax * p.tmax / (2.0 * pmin * pmin);
+    const bool fast = qb * (double)nb < 1073741824.0;  // 2^30
+    const bool fast32 = fast && qb < 524288.0;         // and |q| < 2^19: one FMA
+
+    auto exact_bin = [&](double td, int c) -> uint32_t {
+        return fpw_ref_bin(period_dt != 0.0f ? fold_exact<true>(td, s[c])
+                                             : fold_exact<false>(td, s[c]),
+                           p);
+    };
+    // Beyond the one-FMA range: floor(q' n_bins) - n_bins floor(q') from a
+    // round-down floor and one round-down FMA with 20 fraction bits.
+    auto wide_bin = [&](double td, int c) -> uint32_t {
+        if (fast) {
+            const double a = period_dt != 0.0f ? td - s[c].c * td * td : td;
+            const double qh = __dmul_rn(a, s[c].yhi);
+            const double r = __dadd_rd(qh, kMagic15);
+            const double y = __fma_rd(qh, (double)nb * 1048576.0, kMagic15);
+            const uint32_t ylo = (uint32_t)__double2loint(y);
+            // biased by 2^31 by the magic constant's top mantissa bit
+            const uint32_t b = __funnelshift_r(ylo, (uint32_t)__double2hiint(y), 20) +
+                               (uint32_t)__double2loint(r) * (0u - nb) - 0x80000000u;
+            if (ylo * 4096u + (p.edge_d << 12) >= ((2u * p.edge_d) << 12)) return b;
+        }
+        return exact_bin(td, c);
+    };
+
+    auto run = [&](auto pdt_tag, auto f32_tag) {
+        constexpr bool HAS_PDT = decltype(pdt_tag)::value;
+        constexpr bool F32 = decltype(f32_tag)::value;
+        double y32[CELLS], pc[CELLS];
+#pragma unroll
+        for (int c = 0; c < CELLS; c++) {
+            y32[c] = s[c].yhi * 4294967296.0;  // RN(1/P) * 2^32, exact
+            pc[c] = s[c].c;
+        }
+        // G points from i: their bins, then their updates.
+        auto group = [&](auto g_tag, uint32_t i) {
+            constexpr int G = decltype(g_tag)::value;
+            Point q[G];
+            uint32_t b[G][CELLS];
+#pragma unroll
+            for (int k = 0; k < G; k++) q[k] = st[i + k];
+            if constexpr (F32) {
+                uint32_t lo[G][CELLS], least = 0xFFFFFFFFu;
+#pragma unroll
+                for (int k = 0; k < G; k++)
+#pragma unroll
+                    for (int c = 0; c < CELLS; c++) {
+                        double a = q[k].t;
+                        if constexpr (HAS_PDT) a = q[k].t - pc[c] * q[k].t * q[k].t;
+                        const double y = __fma_rd(a, y32[c], p.magic32);
+                        mul_wide_u32((uint32_t)__double2loint(y), nb, lo[k][c], b[k][c]);
+                        least = min(least, lo[k][c]);
+                    }
+                if (least < p.edge32_lim) {
+#pragma unroll
+                    for (int k = 0; k < G; k++)
+#pragma unroll
+                        for (int c = 0; c < CELLS; c++)
+                            if (lo[k][c] < p.edge32_lim) b[k][c] = exact_bin(q[k].t, c);
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < G; k++)
+#pragma unroll
+                    for (int c = 0; c < CELLS; c++) b[k][c] = wide_bin(q[k].t, c);
+            }
+#pragma unroll
+            for (int k = 0; k < G; k++) {
+                float2 x[CELLS];
+#pragma unroll
+                for (int c = 0; c < CELLS; c++) x[c] = ld(b[k][c] + kRow0, c);
+#pragma unroll
+                for (int c = 0; c < CELLS; c++) {
+                    x[c].x += q[k].iv;
+                    x[c].y += q[k].ivy;
+                }
+#pragma unroll
+                for (int c = 0; c < CELLS; c++) put(b[k][c] + kRow0, c, x[c]);
+            }
+        };
+        for (uint32_t base = 0; base < n; base += kFpwTile) {
+            const uint32_t cnt = min(kFpwTile, n - base);
+            __syncthreads();
+            for (uint32_t i = tid; i < cnt; i += BLOCK)
+                st[i] = Point{(double)p.t[off + base + i], p.iv[off + base + i],
+                              p.ivy[off + base + i]};
+            __syncthreads();
+            if (!active) continue;
+            constexpr int kG = F32 ? 4 : 1;
+            uint32_t i = 0;
+#pragma unroll 1
+            for (; i + kG <= cnt; i += kG) group(std::integral_constant<int, kG>{}, i);
+#pragma unroll 1
+            for (; i < cnt; i++) group(std::integral_constant<int, 1>{}, i);
+        }
+    };
+    using T_ = std::true_type;
+    using F_ = std::false_type;
+    if (!fast32) run(F_{}, F_{});  // the wide bin tests the derivative itself
+    else if (period_dt != 0.0f) run(T_{}, T_{});
+    else run(F_{}, T_{});
+
+    if (!active) return;
+    float acc[CELLS];
+    if constexpr (BLS) {
+        bls_values<CELLS>(ld, put, nb, p.nb_min, p.nb_max, acc);
+    } else {
+#pragma unroll
+        for (int c = 0; c < CELLS; c++)
+            acc[c] = fpw_value([&](uint32_t k) { return ld(k, c); }, nb);
+    }
+#pragma unroll
+    for (int c = 0; c < CELLS; c++) {
+        const uint64_t pi = pi0 + (uint64_t)c * BLOCK;
+        if (pi < p.n_per)
+            p.out[cv * (p.n_per * p.n_pdt) + pi * p.n_pdt + dt] = acc[c];
+    }
 }
 
 }  // namespace PF_KNS

@@ -105,6 +105,8 @@ struct FpwParams {
     float* out;
     double tmax;      // max |t| over the batch (the chosen form's range guard)
     uint32_t edge_d;  // bin-edge guard, units of 2^-20 bin (as the CE / AOV bin kernels)
+    double magic32;   // and the one-FMA bin's constants (FoldParams)
+    uint32_t edge32_lim;
     int bls;          // BLS instead of FPW (ivy then holds w * (m - weighted mean))
     uint32_t nb_min, nb_max;  // BLS: window widths searched, in bins
 };
