@@ -43,15 +43,17 @@
 //     point is its time alone and the counter word and increment stay in
 //     registers for a column's run;
 //   - a thread holds CELLS = 2 periods, so one load serves two evaluations
-//     (4 were slower: 96-128 registers at 10 warps per SM);
+//     (4 were slower: 96-128 registers at 10 warps per SM; so was staging the
+//     times as floats and converting each, 5-7%: the conversions take the XU
+//     pipe);
 //   - the guard rides in the FMA's constant and the product is one wide
 //     multiply, so an evaluation is DFMA, IMAD.WIDE, IMAD, RED and half a
 //     three-way minimum (6.4 instructions with all overheads on 4096 points,
 //     11.1 before).
 // Measured, 3000 ragged curves (20-2000 points) x 20000 periods, CE 10 x 10
 // then AOV 15, plan with peaks: 12.06 -> 10.40 ms and 11.63 -> 8.99 ms (9.57
-// and 8.86 ms with the statistics below); CE 200 x 4096 x 10000 x 2
-// derivatives 7.26 -> 5.18 ms.  CE [1024,4096):
+// and 8.86 ms with the statistics below, CE 9.09 with their table); CE 200 x
+// 4096 x 10000 x 2 derivatives 7.26 -> 5.14 ms.  CE [1024,4096):
 // issue 61%, fmaheavy pipe 73%, shared-memory pipe 50%; AOV: shared-memory
 // pipe 88% (its two reductions per evaluation).
 #pragma once
@@ -94,6 +96,10 @@ __device__ __forceinline__ uint32_t lds_u32(uint32_t addr) {
 }
 
 constexpr double kMagic15 = 6755399441055744.0;  // 1.5 * 2^52
+
+// Curves shorter than this take the CE statistic's logs from a table.
+constexpr uint32_t kXlxTable = 512;
+static_assert(kXlxTable * 4 <= kBinTile * 8, "the table takes the staged tile's place");
 
 // A staged point of the shared-histogram kernel (pf_binwarp.cuh): its time,
 // and its magnitude bin (CE) or fixed-point magnitude (AOV).
@@ -150,10 +156,27 @@ __device__ __forceinline__ float aov_finish(double sbx, double xx_n, double sumx
 // the log's 110 operations per cell on the XU pipe).  8-bit counters for
 // curves under 256 points, which double the resident warps, were slower
 // (1.15 -> 1.18 ms).
-template <bool CNT16, int CELLS>
+//
+// TABLE: c log2 c comes from a table in shared memory at `table` (byte c * 4;
+// the same ce_xlx values) and the counters count in units of 4, so that a
+// counter is the table's byte offset: two operations per count instead of
+// six, and none on the XU pipe.  Small counts fall on different banks or on
+// the same word, so the lookups hardly conflict.  Samples: [64,256) 1.15 -> 1.05
+// ms, [256,1024) 0.70 -> 0.65; CE of 3000 ragged curves x 20000 periods 9.57 ->
+// 9.09 ms.
+__device__ __forceinline__ float lds_f32(uint32_t addr) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+    return v;
+}
+template <bool CNT16, int CELLS, bool TABLE>
 __device__ __forceinline__ void ce_stat_fast(uint32_t tbase, uint32_t cell_bytes, uint32_t nP,
                                              uint32_t W, uint32_t cols, uint32_t n,
-                                             float (&out)[CELLS]) {
+                                             uint32_t table, float (&out)[CELLS]) {
+    auto xlx = [&](uint32_t c) -> float {
+        if constexpr (TABLE) return lds_f32(table + c);
+        else return ce_xlx(c);
+    };
     float acc[CELLS];
 #pragma unroll
     for (int c = 0; c < CELLS; c++) acc[c] = 0.0f;
@@ -177,11 +200,10 @@ __device__ __forceinline__ void ce_stat_fast(uint32_t tbase, uint32_t cell_bytes
                 for (int c = 0; c < CELLS; c++) {
                     const uint32_t wv = lds_u32(at + r * (cols * 4u) + c * cell_bytes);
                     // Both 16-bit halves summed at once: each half's total
-                    // is at most n < 2^16, so no carry crosses halves.
+                    // is below 2^16, so no carry crosses halves.
                     col[r][c] += wv;
                     row[r][c] = __fadd_rn(
-                        row[r][c], CNT16 ? __fadd_rn(ce_xlx(wv & 0xFFFFu), ce_xlx(wv >> 16))
-                                         : ce_xlx(wv));
+                        row[r][c], CNT16 ? __fadd_rn(xlx(wv & 0xFFFFu), xlx(wv >> 16)) : xlx(wv));
                 }
         }
 #pragma unroll
@@ -189,7 +211,7 @@ __device__ __forceinline__ void ce_stat_fast(uint32_t tbase, uint32_t cell_bytes
 #pragma unroll
             for (int c = 0; c < CELLS; c++) {
                 const uint32_t t = CNT16 ? (col[r][c] & 0xFFFFu) + (col[r][c] >> 16) : col[r][c];
-                acc[c] = __fadd_rn(acc[c], __fsub_rn(ce_xlx(t), row[r][c]));
+                acc[c] = __fadd_rn(acc[c], __fsub_rn(xlx(t), row[r][c]));
             }
     };
     uint32_t j = 0;
@@ -345,8 +367,12 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
             reinterpret_cast<double2*>(tile_t)[2 * i4 + 1] = make_double2(q.z, q.w);
         }
     };
+    // CE statistic by table (ce_stat_fast) where the table fits the staged
+    // tile's place, which it takes after the round's last point.
+    const bool table = ALGO == ALGO_CE && !REF_STATS && CNT16 && n < kXlxTable;
+    const uint32_t unit = table ? 4u : 1u;
     // A curve that fits one tile is staged once for every round.
-    const bool one_tile = n_pad <= kBinTile;
+    const bool one_tile = n_pad <= kBinTile && !(table && ROUNDS > 1);
     if (one_tile) {
         __syncthreads();
         stage(0, n_pad);
@@ -590,7 +616,7 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
                     const uint32_t word = CNT16 ? col >> 1 : col;
                     if (hi > lo)
                         span(lo - base, hi - lo, tbase + word * (nP * kCols * 4),
-                             (CNT16 && (col & 1u)) ? 0x10000u : 1u);
+                             (CNT16 && (col & 1u)) ? unit << 16 : unit);
                     const uint32_t next_at = run_at + ((len + 3u) & ~3u);
                     if (next_at > end) break;  // the rest lies in the next tile
                     run_at = next_at;
@@ -616,10 +642,21 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
     compiler_fence();
     __syncwarp();
     if constexpr (!REF_STATS) {
+        if (table) {  // uniform over the CTA
+            __syncthreads();
+            for (uint32_t c = tid; c <= n; c += BLOCK)
+                reinterpret_cast<float*>(tile_t)[c] = ce_xlx(c);
+            __syncthreads();
+        }
         if (active) {
             float res[CELLS];
             if constexpr (ALGO == ALGO_CE) {
-                ce_stat_fast<CNT16, CELLS>(tbase, BLOCK * 4, nP, W, kCols, n, res);
+                if (table)
+                    ce_stat_fast<CNT16, CELLS, true>(
+                        tbase, BLOCK * 4, nP, W, kCols, n,
+                        (uint32_t)__cvta_generic_to_shared(tile_t), res);
+                else
+                    ce_stat_fast<CNT16, CELLS, false>(tbase, BLOCK * 4, nP, W, kCols, n, 0u, res);
             } else {
                 double sbx[CELLS];
                 aov_sbx_fast<CELLS>(tbase, BLOCK * 4, nP, kCols, sbx);
