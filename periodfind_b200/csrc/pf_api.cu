@@ -885,7 +885,8 @@ cudaError_t launch_fold_sem(const Job& j, const FoldConfig& c, const FoldParams&
 
 // Launch shape of one length class.  Cached per context; the first time a
 // key is met, every candidate (the bin kernel: block 32 / 64 / 128 where
-// shared memory allows, 1 or 2 periods per thread at once, in 1 or 4 rounds;
+// shared memory allows, 1 or 2 periods per thread at once (AOV also 3 at block
+// 64), in 1 or 4 rounds;
 // the others: block 64 / 128 / 256, persistent or one CTA per item) is timed
 // with CUDA events on a
 // sample of the class (a contiguous run of its curves from the middle of
@@ -968,8 +969,9 @@ int tuned_config(pf_ctx* ctx, const Job& j, const FoldConfig& base, int cls, uin
             if (block == (bin ? 256 : 32)) continue;
             FoldConfig t = base;
             t.block = block;
-            for (int cells : {1, 2}) {
+            for (int cells : {1, 2, 3}) {
                 if (!bin && cells > 1) continue;
+                if (cells == 3 && !(base.algo == ALGO_AOV && block == 64)) continue;
                 t.cells = cells;
                 if (fold_smem(t, j.n_phase, j.n_mag) > ctx->smem_optin) continue;
                 // bin kernel: 1 or 4 rounds; others: persistent or not

@@ -42,10 +42,11 @@
 //   - CE takes its points sorted by magnitude column (ce_sort_kernel), so a
 //     point is its time alone and the counter word and increment stay in
 //     registers for a column's run;
-//   - a thread holds CELLS = 2 periods, so one load serves two evaluations
-//     (4 were slower: 96-128 registers at 10 warps per SM; so was staging the
-//     times as floats and converting each, 5-7%: the conversions take the XU
-//     pipe);
+//   - a thread holds CELLS = 2 periods, for AOV also 3, so one load serves as
+//     many evaluations (AOV samples from 256 points on 0.64 -> 0.60 ms with 3;
+//     CE 10% slower with 3, both slower with 4: too few warps); staging the
+//     times as floats and converting each was 5-7% slower, as the conversions
+//     take the XU pipe;
 //   - the guard rides in the FMA's constant and the product is one wide
 //     multiply, so an evaluation is DFMA, IMAD.WIDE, IMAD, RED and half a
 //     three-way minimum (6.4 instructions with all overheads on 4096 points,
@@ -63,10 +64,10 @@ namespace PF_KNS {
 
 // Resident CTAs per SM the bin kernel is compiled for: 1024 cells (CE, the
 // shared-memory limit of 10 x 10 counters) and 1280 (AOV; 1024 measured 2-3%
-// slower) per SM.
+// slower), 1536 with three cells per thread, per SM.
 template <int ALGO, int BLOCK, int CELLS>
 constexpr int bin_min_blocks() {
-    return (ALGO == ALGO_CE ? 1024 : 1280) / (BLOCK * CELLS);
+    return (ALGO == ALGO_CE ? 1024 : CELLS == 3 ? 1536 : 1280) / (BLOCK * CELLS);
 }
 
 // Fire-and-forget shared reduction.  No "memory" clobber: the counters it

@@ -44,7 +44,7 @@ struct FoldConfig {
                     // one CTA per item
     int rounds;     // bin kernel: an item is rounds x cells x block periods (1 or 4);
                     // KIND_LSREC: frequencies per thread (4 or 8)
-    int cells;      // bin kernel: periods a thread holds at once (1 or 2)
+    int cells;      // bin kernel: periods a thread holds at once (1, 2 or, AOV, 3)
     int n_sm;       // persistent kernels: grid = n_sm x resident CTAs per SM
 };
 
