@@ -71,7 +71,8 @@
  *                  one sine / cosine per point and thread followed by
  *                  angle-addition rotations along the uniform grid, or a
  *                  non-uniform FFT of the points (blocks of 4096
- *                  frequencies; a candidate from 1024 frequencies on).
+ *                  frequencies; a candidate from 1024 frequencies and 64
+ *                  points on).
  *  PF_BINS_SHARED  (CE / AOV, chosen) keep the shared-histogram binning
  *                  (one histogram per warp and trial period, filled with
  *                  shared atomics) for the length classes it serves (curves

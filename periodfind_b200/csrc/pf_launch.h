@@ -134,7 +134,7 @@ struct NufftParams {
     const float* m;
     const CurveDesc* curves;
     const uint32_t* order;
-    const float* deconv;  // launch_nufft_deconv's table
+    const float* table;   // launch_nufft_table's
     uint32_t n_freq;
     uint32_t blocks;      // per curve
     double f0, df;
@@ -145,8 +145,9 @@ struct NufftParams {
 // this fraction of n^2 (n^2 / 4 for well spread phases).
 constexpr float kNufftSingular = 1e-3f;
 cudaError_t launch_nufft(const NufftParams& p, uint32_t n_curves, cudaStream_t s);
-// The kernel transform's inverse, kNufftModes / 2 + 1 floats.
-cudaError_t launch_nufft_deconv(float* deconv, cudaStream_t s);
+// Twiddles and deconvolution factors.
+constexpr int kNufftTableFloats = 4 * kNufftModes + kNufftModes / 2 + 1;
+cudaError_t launch_nufft_table(float* table, cudaStream_t s);
 
 // Preparation kernels (pf_prep.cu).
 // max |t| over n packed points into *tmax_bits (float bits; zeroed first).

@@ -27,8 +27,8 @@
 // for 83 curves of 4096-16384 points x 50000 frequencies.)
 //
 // Measured, 300 curves of 64-16384 points x 50000 frequencies: 14.95 ms with
-// the recurrence, 1.02 ms with this form; error of the power against FP64
-// 6.1e-6 and 5.0e-7 (2-norm).  Bound: short curves by the FFTs (about 29000 SM
+// the recurrence, 1.13 ms with this form; error of the power against FP64
+// 6.8e-6 and 3.7e-7 (2-norm).  Bound: short curves by the FFTs (about 29000 SM
 // cycles a block: barriers and shared memory), long ones by the spreading's
 // issue slots (staging arithmetic, 16 reductions per point and sum).  The
 // direct sums stay for grids below kNufftMinFreqs and where they are faster
@@ -111,8 +111,12 @@ __device__ __forceinline__ void fft16(float2 (&v)[16]) {
 // One radix-16 pass of the self-sorting FFT over the grid: sub-transforms of
 // length NS become ones of length 16 NS.  The first (NS = 1) takes its input
 // in v, the others from the grid.
+// Twiddles come from a table of e^{2 pi i k / kM} rounded from FP64: six of a
+// pass's fifteen are read, the others are one product of two of them (powers
+// of the first by repeated products cost a fifth of the result's accuracy).
 template <int NS>
-__device__ __forceinline__ void pass16(Smem& sm, float2 (&v)[16]) {
+__device__ __forceinline__ void pass16(Smem& sm, const float2* __restrict__ tw,
+                                       float2 (&v)[16]) {
     const int tid = threadIdx.x;
     const int q = tid % NS;
     if constexpr (NS > 1) {
@@ -121,13 +125,17 @@ __device__ __forceinline__ void pass16(Smem& sm, float2 (&v)[16]) {
             const int i = pad(tid + r * kThreads);
             v[r] = make_float2(sm.re[i], sm.im[i]);
         }
-        float2 w[16];
-        sincospif(2.0f * (float)q / (float)(16 * NS), &w[1].y, &w[1].x);
-        v[1] = cmul(v[1], w[1]);
+        constexpr int kStep = kM / (16 * NS);
+        float2 w[4], w4[4];
 #pragma unroll
-        for (int r = 2; r < 16; r++) {
-            w[r] = (r & 1) ? cmul(w[r - 1], w[1]) : cmul(w[r / 2], w[r / 2]);
-            v[r] = cmul(v[r], w[r]);
+        for (int r = 1; r < 4; r++) {
+            w[r] = __ldg(tw + q * r * kStep);
+            w4[r] = __ldg(tw + q * 4 * r * kStep);
+        }
+#pragma unroll
+        for (int r = 1; r < 16; r++) {
+            const float2 f = r < 4 ? w[r & 3] : (r & 3) ? cmul(w4[r >> 2], w[r & 3]) : w4[r >> 2];
+            v[r] = cmul(v[r], f);
         }
     }
     fft16(v);
@@ -147,7 +155,8 @@ __device__ __forceinline__ void pass16(Smem& sm, float2 (&v)[16]) {
 // one.  MULT = 1: S (values y); MULT = 2: Q (values 1).  `scale` turns
 // a value into grid units.
 template <int MULT>
-__device__ __forceinline__ void spread_and_transform(Smem& sm, const float* __restrict__ t,
+__device__ __forceinline__ void spread_and_transform(Smem& sm, const float2* __restrict__ tw,
+                                                     const float* __restrict__ t,
                                                      const float* __restrict__ y, uint32_t n,
                                                      double fc, double df, float scale) {
     const int tid = threadIdx.x;
@@ -186,8 +195,10 @@ __device__ __forceinline__ void spread_and_transform(Smem& sm, const float* __re
 #pragma unroll
             for (int l = 0; l < kW; l++) {
                 const float z = ((float)(l - (kW / 2 - 1)) - fr) * (2.0f / kW);
-                const float r = sqrtf(fmaxf(1.0f - z * z, 0.0f));
-                const float w = __expf(kBeta * (r - 1.0f));
+                // beta (sqrt(1 - z^2) - 1) without the cancellation near z = 0
+                const float zz = z * z;
+                const float r = sqrtf(fmaxf(1.0f - zz, 0.0f));
+                const float w = __expf(__fdividef(-kBeta * zz, 1.0f + r));
                 const int i = pad((first + l) & (kM - 1));
                 atomicAdd(&gre[i], __float2int_rn(c * w));
                 atomicAdd(&gim[i], __float2int_rn(s * w));
@@ -207,18 +218,17 @@ __device__ __forceinline__ void spread_and_transform(Smem& sm, const float* __re
         }
         __syncthreads();
     }
-    pass16<1>(sm, v);
-    pass16<16>(sm, v);
-    pass16<256>(sm, v);
+    pass16<1>(sm, tw, v);
+    pass16<16>(sm, tw, v);
+    pass16<256>(sm, tw, v);
 }
 
 // Mode of index j (0 <= j < kM / 2) after the radix-16 passes: kappa = j for
 // j < kM / 4, else j - kM / 2 (the last pass gives two modes per j, of which
 // exactly one lies in the kept half).
-__device__ __forceinline__ float2 mode(const Smem& sm, int j) {
+__device__ __forceinline__ float2 mode(const Smem& sm, const float2* __restrict__ tw, int j) {
     const int a = pad(j), b = pad(j + kM / 2);
-    float2 w;
-    sincospif(2.0f * (float)j / (float)kM, &w.y, &w.x);
+    const float2 w = __ldg(tw + j);
     const float2 x = make_float2(sm.re[a], sm.im[a]);
     const float2 z = cmul(make_float2(sm.re[b], sm.im[b]), w);
     return j < kM / 4 ? cadd(x, z) : csub(x, z);
@@ -233,6 +243,8 @@ __global__ void __launch_bounds__(kThreads, 2)
     const CurveDesc cd = p.curves[c];
     const float* t = p.t + cd.off;
     const float* y = p.m + cd.off;
+    const float2* tw = reinterpret_cast<const float2*>(p.table);
+    const float* deconv = p.table + 2 * kM;
     const uint32_t n = cd.n;
     if (p.stamps && threadIdx.x == 0) p.stamps[2 * (size_t)blockIdx.x] = global_ns();
     const double fc = p.f0 + (double)(k0 + kNufftModes / 2) * p.df;
@@ -254,18 +266,19 @@ __global__ void __launch_bounds__(kThreads, 2)
     if ((threadIdx.x & 31) == 0) atomicMax(&s_max, my_max);
     bad = __syncthreads_or(bad ? 1 : 0) != 0;
     const float y_max = __uint_as_float(s_max);
-    constexpr float kFull = 2147483392.0f / kTilePts;  // below 2^31 / kTilePts
+    // Grid units per largest value: a tile's sum stays below 2^31.
+    const float full = 2147483392.0f / (float)min(max(n, 1u), (uint32_t)kTilePts);
     // (squares below 1e-60 are zero in the direct sums too)
-    const float y_scale = y_max > 1e-30f ? kFull / y_max : 0.0f;
+    const float y_scale = y_max > 1e-30f ? full / y_max : 0.0f;
     const float nan = __uint_as_float(0x7FC00000u);
-    const float y_unit = bad ? nan : y_max * (1.0f / kFull), q_unit = bad ? nan : 1.0f / kFull;
+    const float y_unit = bad ? nan : y_max / full, q_unit = bad ? nan : 1.0f / full;
 
     float2 q[kPer];
-    spread_and_transform<2>(sm, t, y, n, fc, p.df, kFull);
+    spread_and_transform<2>(sm, tw, t, y, n, fc, p.df, full);
 #pragma unroll
-    for (int i = 0; i < kPer; i++) q[i] = mode(sm, threadIdx.x + i * kThreads);
+    for (int i = 0; i < kPer; i++) q[i] = mode(sm, tw, threadIdx.x + i * kThreads);
     __syncthreads();
-    spread_and_transform<1>(sm, t, y, n, fc, p.df, y_scale);
+    spread_and_transform<1>(sm, tw, t, y, n, fc, p.df, y_scale);
 
     float* out = p.out + (size_t)c * p.n_freq;
     unsigned again = 0;  // the thread's near-singular modes
@@ -275,8 +288,8 @@ __global__ void __launch_bounds__(kThreads, 2)
         const int kappa = j < kM / 4 ? j : j - kM / 2;
         const uint64_t k = (uint64_t)k0 + (uint32_t)(kappa + kNufftModes / 2);
         if (k >= p.n_freq) continue;
-        const float dc = p.deconv[kappa < 0 ? -kappa : kappa];
-        const float2 sv = mode(sm, j);
+        const float dc = deconv[kappa < 0 ? -kappa : kappa];
+        const float2 sv = mode(sm, tw, j);
         const float dy = dc * y_unit, dq = dc * q_unit;
         const LSAcc a{sv.x * dy, sv.y * dy, 0.5f * fmaf(q[i].x, dq, (float)n),
                       0.5f * q[i].y * dq};
@@ -321,10 +334,16 @@ __global__ void __launch_bounds__(kThreads, 2)
     if (p.stamps && threadIdx.x == 0) p.stamps[2 * (size_t)blockIdx.x + 1] = global_ns();
 }
 
-// 1 / (the kernel's transform at mode k), k = 0 .. kNufftModes / 2: the
-// trapezoidal rule on the even kernel, which has all but vanished at its ends.
-__global__ void nufft_deconv_kernel(float* __restrict__ deconv) {
+// The table: e^{2 pi i k / kM} for k < kM, then 1 / (the kernel's transform at
+// mode k) for k <= kNufftModes / 2 (the trapezoidal rule on the even kernel,
+// which has all but vanished at its ends).
+__global__ void nufft_table_kernel(float* __restrict__ table) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= kM) return;
+    double sn, cs;
+    sincospi(2.0 * (double)k / kM, &sn, &cs);
+    table[2 * k] = (float)cs;
+    table[2 * k + 1] = (float)sn;
     if (k > kNufftModes / 2) return;
     constexpr int kNodes = 96;
     double sum = 0.5;  // half the value at z = 0
@@ -333,13 +352,14 @@ __global__ void nufft_deconv_kernel(float* __restrict__ deconv) {
         sum += exp((double)kBeta * (sqrt(1.0 - z * z) - 1.0)) *
                cospi((double)k * kW * z / (double)kM);
     }
-    deconv[k] = (float)(1.0 / (sum * kW / kNodes));
+    table[2 * kM + k] = (float)(1.0 / (sum * kW / kNodes));
 }
 
 }  // namespace PF_KNS
 
-cudaError_t launch_nufft_deconv(float* deconv, cudaStream_t s) {
-    PF_KNS::nufft_deconv_kernel<<<(kNufftModes / 2 + 64) / 64, 64, 0, s>>>(deconv);
+cudaError_t launch_nufft_table(float* table, cudaStream_t s) {
+    static_assert(kNufftTableFloats == 2 * PF_KNS::kM + kNufftModes / 2 + 1, "table size");
+    PF_KNS::nufft_table_kernel<<<PF_KNS::kM / 64, 64, 0, s>>>(table);
     return cudaGetLastError();
 }
 

@@ -100,7 +100,7 @@ struct FoldParams {
     // derivative, 0.
     int fgrid;
     double f0, df;
-    const float* nufft_deconv;  // the non-uniform FFT's table (pf_nufft.cu)
+    const float* nufft_table;  // the non-uniform FFT's table (pf_nufft.cu)
 };
 
 // Staged points of the chosen bin kernel: the time as a double, for AOV also
