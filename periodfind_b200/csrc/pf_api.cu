@@ -629,6 +629,12 @@ FoldConfig choose_config(pf_ctx* ctx, const Job& j, uint32_t max_len, bool& ok) 
         c.acc = AOVACC_FIX;
     }
     ok = false;
+    // The largest histogram a call may ask for: 64 columns of counters beside
+    // 4 KB of staged points (the smaller CTAs below would fit larger ones).
+    if (c.kind == KIND_BIN &&
+        bin_smem_bytes(c.algo, c.cnt16, 64, j.n_phase, j.n_mag) - bin_tile_bytes(c.algo) + 4096 >
+            ctx->smem_optin)
+        return c;
     if (c.kind == KIND_BIN && !c.ref_stats) {
         // Without tuning: two periods per thread in small CTAs (the shape
         // tuning mostly picks), fewer where the histograms are large.
