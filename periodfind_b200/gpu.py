@@ -517,8 +517,10 @@ class LombScargle(_Periodogram):
         On a uniform frequency grid the phase of a point advances by the same
         angle from one frequency to the next, so the sine and cosine can
         follow the grid by angle-addition rotations instead of one MUFU pair
-        per evaluation.  trig: None lets the autotuner pick per curve-length
-        class; 'sincos' or 'recurrence' keeps one form.  Chosen form and
+        per evaluation, and the sums of a whole block of frequencies follow
+        from one non-uniform FFT.  trig: None lets the autotuner pick per
+        curve-length class; 'sincos' or 'recurrence' keeps one form.  Chosen
+        form and
         CUDA arithmetic only (fold='exact' for an FP64 phase)."""
         if self.mode != "chosen" or self.semantics != "cuda":
             raise ValueError("a frequency grid needs mode='chosen', semantics='cuda'")
