@@ -415,13 +415,26 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
         }
         if (!active) continue;
 
+        // t_corr = t - c t^2 for the fast bins.  AOV takes it in one FMA from
+        // the point's square, which is exact (t has 24 bits) and which the
+        // thread's cells share (250 x 4096 points x 10000 periods x 2
+        // derivatives with peaks: 8.40 -> 8.03 ms).  It differs from the
+        // reference's by its rounding of c t: |c t^2 / P| n 2^-53 <= 2^-23 of a
+        // bin while |q| n < 2^30, which the guard's two units of 2^-20 cover;
+        // the exact sequence keeps the reference's order.  CE keeps that order
+        // here too: its groups of 16 points have no register left for the
+        // squares (4 % gained with a derivative, 1 % lost to spills without).
+        auto t_corr = [&](double td, double c_) -> double {
+            if constexpr (ALGO == ALGO_AOV) return __fma_rn(-c_, __dmul_rn(td, td), td);
+            else return td - c_ * td * td;
+        };
         // Fast bin of one point: row (+2^31 bias) and the edge-test value
         // ((fraction + D) << 12); the point is near an edge iff ev < edge_lim.
         auto fast_bin = [&](double td, double y_, double c_, auto has_pdt_tag,
                             uint32_t& ev) -> uint32_t {
             constexpr bool HAS_PDT = decltype(has_pdt_tag)::value;
             double a = td;
-            if constexpr (HAS_PDT) a = td - c_ * td * td;
+            if constexpr (HAS_PDT) a = t_corr(td, c_);
             const double qh = __dmul_rn(a, y_);
             const double r = __dadd_rd(qh, kMagic15);
             const double y = __fma_rd(qh, nd20, kMagic15);
@@ -444,7 +457,7 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
                               uint32_t& ev) -> uint32_t {
             constexpr bool HAS_PDT = decltype(has_pdt_tag)::value;
             double a = td;
-            if constexpr (HAS_PDT) a = td - c_ * td * td;
+            if constexpr (HAS_PDT) a = t_corr(td, c_);
             const double y = __fma_rd(a, y32, p.magic32);
             const uint32_t f = (uint32_t)__double2loint(y);
             uint32_t row;
@@ -537,8 +550,12 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
                     for (int c = 0; c < CELLS; c++)
 #pragma unroll
                         for (int k = 0; k < G; k++) {
+                            // (a square kept for here would cost registers)
+                            double t = td[k];
+                            if constexpr (ALGO == ALGO_AOV && decltype(has_pdt_tag)::value)
+                                asm("" : "+d"(t));
                             uint32_t ev;
-                            bin_of(td[k], ys[c], pc[c], ev);
+                            bin_of(t, ys[c], pc[c], ev);
                             if (ev < lim) near |= 1u << (c * G + k);
                         }
                     if constexpr (MASK) {

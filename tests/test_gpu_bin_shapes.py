@@ -69,3 +69,22 @@ def test_ce_many_columns_and_short_curves():
     got = ConditionalEntropy(2, 400, semantics="cpu").periodograms(ts, ms, periods, pdts)
     want = O.ce(ts, ms, periods, pdts, 2, 400)
     np.testing.assert_allclose(got, want, rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("span,pdt", [(900.0, 1e-3), (900.0, -0.05), (30000.0, 2e-4)])
+@pytest.mark.parametrize("n_phase", [2, 15, 40])
+def test_aov_bins_with_strong_derivatives(span, pdt, n_phase):
+    """Period derivatives whose correction is larger than the time itself or
+    nearly cancels it: every bin count equal to the reference's."""
+    from periodfind_b200.gpu import AOV
+
+    rng = np.random.default_rng(n_phase)
+    ts = [lc.uniform_times(rng, n, span) for n in (7, 257, 1000)]
+    ms = [rng.random(len(t)).astype(np.float32) for t in ts]
+    periods = np.geomspace(0.07, 40.0, 131).astype(np.float32)
+    pdts = np.array([pdt], np.float32)
+    _, got = AOV(n_phase, mode="chosen", semantics="cpu").bin_counts(ts, ms, periods, pdts)
+    for c, (t, m) in enumerate(zip(ts, ms)):
+        for i, P in enumerate(periods):
+            _, want = O.aov_counts(t, m, P, pdts[0], n_phase)
+            np.testing.assert_array_equal(got[c, i, 0], want)
