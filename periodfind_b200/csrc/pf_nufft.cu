@@ -266,8 +266,11 @@ __global__ void __launch_bounds__(kThreads, 2)
     if ((threadIdx.x & 31) == 0) atomicMax(&s_max, my_max);
     bad = __syncthreads_or(bad ? 1 : 0) != 0;
     const float y_max = __uint_as_float(s_max);
-    // Grid units per largest value: a tile's sum stays below 2^31.
-    const float full = 2147483392.0f / (float)min(max(n, 1u), (uint32_t)kTilePts);
+    // Grid units per largest value.  A tile's sum stays below 2^31 where all of
+    // its points fall into one cell at phase 0: 2^13 below it, for half a unit
+    // of rounding per point (2^8 in all) and a few 2^-24 of the scale, the sine
+    // and the weight (under 2^12).
+    const float full = 2147475456.0f / (float)min(max(n, 1u), (uint32_t)kTilePts);
     // (squares below 1e-60 are zero in the direct sums too)
     const float y_scale = y_max > 1e-30f ? full / y_max : 0.0f;
     const float nan = __uint_as_float(0x7FC00000u);
