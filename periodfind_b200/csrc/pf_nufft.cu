@@ -250,8 +250,9 @@ __global__ void __launch_bounds__(kThreads, 2)
     const double fc = p.f0 + (double)(k0 + kNufftModes / 2) * p.df;
     constexpr int kPer = kNufftModes / kThreads;  // modes per thread
 
-    // Largest |y|; a point that is not finite makes every value NaN, as in
-    // the direct sums.
+    // Largest |y|.  A point that is not finite makes every power NaN, as in the
+    // direct form (an infinite sum is so with one sign in one of the two terms
+    // and the other in the other): written at once, without the transforms.
     __shared__ unsigned s_max;
     if (threadIdx.x == 0) s_max = 0u;
     __syncthreads();
@@ -265,6 +266,14 @@ __global__ void __launch_bounds__(kThreads, 2)
     my_max = __reduce_max_sync(0xffffffffu, my_max);
     if ((threadIdx.x & 31) == 0) atomicMax(&s_max, my_max);
     bad = __syncthreads_or(bad ? 1 : 0) != 0;
+    float* out = p.out + (size_t)c * p.n_freq;
+    if (bad) {
+        const uint32_t k1 = min(k0 + (uint32_t)kNufftModes, p.n_freq);
+        for (uint32_t k = k0 + threadIdx.x; k < k1; k += kThreads)
+            out[k] = __uint_as_float(0x7FC00000u);
+        if (p.stamps && threadIdx.x == 0) p.stamps[2 * (size_t)blockIdx.x + 1] = global_ns();
+        return;
+    }
     const float y_max = __uint_as_float(s_max);
     // Grid units per largest value.  A tile's sum stays below 2^31 where all of
     // its points fall into one cell at phase 0: 2^13 below it, for half a unit
@@ -273,8 +282,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     const float full = 2147475456.0f / (float)min(max(n, 1u), (uint32_t)kTilePts);
     // (squares below 1e-60 are zero in the direct sums too)
     const float y_scale = y_max > 1e-30f ? full / y_max : 0.0f;
-    const float nan = __uint_as_float(0x7FC00000u);
-    const float y_unit = bad ? nan : y_max / full, q_unit = bad ? nan : 1.0f / full;
+    const float y_unit = y_max / full, q_unit = 1.0f / full;
 
     float2 q[kPer];
     spread_and_transform<2>(sm, tw, t, y, n, fc, p.df, full);
@@ -283,7 +291,6 @@ __global__ void __launch_bounds__(kThreads, 2)
     __syncthreads();
     spread_and_transform<1>(sm, tw, t, y, n, fc, p.df, y_scale);
 
-    float* out = p.out + (size_t)c * p.n_freq;
     unsigned again = 0;  // the thread's near-singular modes
 #pragma unroll
     for (int i = 0; i < kPer; i++) {

@@ -31,3 +31,50 @@ def test_every_point_in_one_cell(n, value):
         ts = [t.astype(np.float32)]
         assert np.isnan(_power(ts, ms, f0, df, 2048, "sincos")).all()
         assert np.isnan(_power(ts, ms, f0, df, 2048, "transform")).all()
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_values_that_are_not_finite(bad):
+    """One magnitude that is not finite: NaN at every frequency of its curve, as
+    in the direct form, in no more time than the transform of a clean curve
+    needs (point by point it took 30 times that), and the other curves as before."""
+    import torch
+
+    from periodfind_b200 import _native as nat
+
+    rng = np.random.default_rng(4)
+    n, n_freq, f0, df = 16384, 20000, 0.01, 1e-3
+    ts = [lc.seasonal_times(rng, n, 3000.0).astype(np.float32) for _ in range(8)]
+    ms = [rng.normal(0, 1, n).astype(np.float32) for _ in range(8)]
+    clean = _power(ts, ms, f0, df, n_freq, "transform")
+    spoilt = [m.copy() for m in ms]
+    spoilt[3][77] = bad
+    want = _power(ts, spoilt, f0, df, n_freq, "sincos")
+    got = _power(ts, spoilt, f0, df, n_freq, "transform")
+    np.testing.assert_array_equal(np.isnan(got), np.isnan(want))
+    assert np.isnan(got[3]).all()
+    np.testing.assert_array_equal(np.delete(got, 3, 0), np.delete(clean, 3, 0))
+
+    off = np.arange(9, dtype=np.int64) * n
+    t = torch.from_numpy(np.concatenate(ts)).cuda()
+    out = torch.empty((8, n_freq), device="cuda")
+    ctx = nat.default_context(0)
+    flags = nat.PF_MODE_CHOSEN | nat.PF_TRIG_TRANSFORM
+
+    def best(mags):
+        m = torch.from_numpy(np.concatenate(mags)).cuda()
+        times = []
+        for _ in range(6):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            stream = torch.cuda.current_stream()
+            a.record()
+            ctx.check(ctx.lib.pf_ls_fgrid_dev(ctx.handle, t.data_ptr(), m.data_ptr(),
+                                              off.ctypes.data, 8, f0, df, n_freq, flags,
+                                              out.data_ptr(), stream.cuda_stream))
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times)
+
+    # (4 times leaves room for clocks and launch gaps; the fault was 34 times.)
+    assert best(spoilt) <= 4.0 * best(ms)
