@@ -20,15 +20,15 @@
 // phase t f_c and t df are good to 1e-11 turns), values, kernel and FFT are
 // FP32.  The spreading is exact in any order, so results are the same from run
 // to run: a tile of at most 512 points is added to the grid with 32-bit integer
-// reductions in units of 2^-31 of 512 times the largest value (2^-23 of one
-// rounding), and then taken into FP32 registers, a thread holding the 16 cells
+// reductions in units of 2^-31 of the sum of its magnitudes, which bounds every
+// cell, and then taken into FP32 registers, a thread holding the 16 cells
 // that its first FFT pass needs.  (Float sums kept in order by giving each
 // cell to one warp were 2.5 times slower on long curves: 1.52 against 0.59 ms
 // for 83 curves of 4096-16384 points x 50000 frequencies.)
 //
 // Measured, 300 curves of 64-16384 points x 50000 frequencies: 14.95 ms with
-// the recurrence, 1.13 ms with this form; error of the power against FP64
-// 6.8e-6 and 3.7e-7 (2-norm).  Bound: short curves by the FFTs (about 29000 SM
+// the recurrence, 1.14 ms with this form; error of the power against FP64
+// 6.8e-6 and 2.5e-7 (2-norm).  Bound: short curves by the FFTs (about 29000 SM
 // cycles a block: barriers and shared memory), long ones by the spreading's
 // issue slots (staging arithmetic, 16 reductions per point and sum).  The
 // direct sums stay for grids below kNufftMinFreqs and where they are faster
@@ -152,16 +152,48 @@ __device__ __forceinline__ void pass16(Smem& sm, const float2* __restrict__ tw,
 
 // Spread one of the two sums' points and transform the grid.  After it, the
 // three radix-16 passes are done and mode(j) below finishes the last, radix-2
-// one.  MULT = 1: S (values y); MULT = 2: Q (values 1).  `scale` turns
-// a value into grid units.
+// one.  MULT = 1: S (values y, |y| <= y_max); MULT = 2: Q (values 1).
 template <int MULT>
 __device__ __forceinline__ void spread_and_transform(Smem& sm, const float2* __restrict__ tw,
                                                      const float* __restrict__ t,
                                                      const float* __restrict__ y, uint32_t n,
-                                                     double fc, double df, float scale) {
+                                                     double fc, double df, float y_max,
+                                                     unsigned (&s_sum)[2]) {
+    // Grid units of a tile: its values' magnitudes sum to less than kRange
+    // units, so no cell reaches 2^31 even where all of them meet in one at
+    // phase 0 (2^13 are left for half a unit of rounding per point and a few
+    // 2^-24 of the scale, the sine and the weight).  A fixed share of the
+    // largest value would hold a curve with one value far off in fewer bits: one
+    // of 85 in 511 points of a 0.3 sinusoid gave a power error of 5.6e-6
+    // (2-norm) against 3.1e-7 and 1.0e-6 of the direct sums.  The magnitudes
+    // are added as integers (s_sum, zero at entry: this tile's and the next
+    // one's), rounded up to 2^-22 of the largest, so that the unit is the same
+    // from run to run.
+    constexpr float kRange = 2147475456.0f;
     const int tid = threadIdx.x;
     int* gre = reinterpret_cast<int*>(sm.re);
     int* gim = reinterpret_cast<int*>(sm.im);
+    // Times come sorted, so neighbouring points land in neighbouring cells: a
+    // tile takes every tiles-th point of the curve, which keeps the lanes of
+    // a warp apart on the grid.
+    const uint32_t tiles = (n + kTilePts - 1) / kTilePts;
+    const uint64_t at0 = (uint64_t)tid * tiles;
+    // (squares of sums of less than 10^8 such values are zero in the direct form)
+    const float per_value = y_max > 1e-27f ? __fdiv_rn(4194304.0f, y_max) : 0.0f;
+    const float per_unit = y_max * 0x1p-22f;
+    float value = 1.0f, scale = 0.0f, unit = 0.0f;
+    auto fetch = [&](uint32_t k) {  // tile k's value, and its part of the sum
+        value = at0 + k < n ? y[at0 + k] : 0.0f;
+        const unsigned sum =
+            __reduce_add_sync(0xffffffffu, __float2uint_ru(fabsf(value) * per_value));
+        if ((tid & 31) == 0) atomicAdd(&s_sum[k & 1u], sum);
+    };
+    if constexpr (MULT == 1) {
+        fetch(0);
+    } else {
+        scale = kRange / (float)min(max(n, 1u), (uint32_t)kTilePts);
+        unit = 1.0f / scale;
+    }
     float2 v[16];
 #pragma unroll
     for (int r = 0; r < 16; r++) {
@@ -171,19 +203,20 @@ __device__ __forceinline__ void spread_and_transform(Smem& sm, const float2* __r
         v[r] = make_float2(0.0f, 0.0f);
     }
     __syncthreads();
-    // Times come sorted, so neighbouring points land in neighbouring cells: a
-    // tile takes every tiles-th point of the curve, which keeps the lanes of
-    // a warp apart on the grid.
-    const uint32_t tiles = (n + kTilePts - 1) / kTilePts;
     for (uint32_t k = 0; k < tiles; k++) {
-        const uint64_t at = (uint64_t)tid * tiles + k;
+        const uint64_t at = at0 + k;
+        if constexpr (MULT == 1) {
+            const float sum = (float)max(s_sum[k & 1u], 1u);
+            scale = fminf(kRange / sum * per_value, 1e38f);
+            unit = sum / kRange * per_unit;
+        }
         if (at < n) {
             const double td = (double)t[at];
             double th = td * (fc * MULT);
             th -= rint(th);
             float s, c;
             sincospif(2.0f * (float)th, &s, &c);
-            const float a = MULT == 1 ? scale * y[at] : scale;
+            const float a = MULT == 1 ? scale * value : scale;
             s *= a;
             c *= a;
             double x = td * (df * MULT);
@@ -204,13 +237,15 @@ __device__ __forceinline__ void spread_and_transform(Smem& sm, const float2* __r
                 atomicAdd(&gim[i], __float2int_rn(s * w));
             }
         }
-        __syncthreads();
         const bool more = k + 1 < tiles;
+        if (MULT == 1 && more) fetch(k + 1);
+        __syncthreads();
+        if (MULT == 1 && tid == 0) s_sum[k & 1u] = 0u;
 #pragma unroll
         for (int r = 0; r < 16; r++) {
             const int i = pad(tid + r * kThreads);
-            v[r].x += (float)gre[i];
-            v[r].y += (float)gim[i];
+            v[r].x = fmaf(unit, (float)gre[i], v[r].x);
+            v[r].y = fmaf(unit, (float)gim[i], v[r].y);
             if (more) {
                 gre[i] = 0;
                 gim[i] = 0;
@@ -253,8 +288,8 @@ __global__ void __launch_bounds__(kThreads, 2)
     // Largest |y|.  A point that is not finite makes every power NaN, as in the
     // direct form (an infinite sum is so with one sign in one of the two terms
     // and the other in the other): written at once, without the transforms.
-    __shared__ unsigned s_max;
-    if (threadIdx.x == 0) s_max = 0u;
+    __shared__ unsigned s_max, s_sum[2];
+    if (threadIdx.x == 0) s_max = s_sum[0] = s_sum[1] = 0u;
     __syncthreads();
     unsigned my_max = 0u;
     bool bad = false;
@@ -275,21 +310,12 @@ __global__ void __launch_bounds__(kThreads, 2)
         return;
     }
     const float y_max = __uint_as_float(s_max);
-    // Grid units per largest value.  A tile's sum stays below 2^31 where all of
-    // its points fall into one cell at phase 0: 2^13 below it, for half a unit
-    // of rounding per point (2^8 in all) and a few 2^-24 of the scale, the sine
-    // and the weight (under 2^12).
-    const float full = 2147475456.0f / (float)min(max(n, 1u), (uint32_t)kTilePts);
-    // (squares below 1e-60 are zero in the direct sums too)
-    const float y_scale = y_max > 1e-30f ? full / y_max : 0.0f;
-    const float y_unit = y_max / full, q_unit = 1.0f / full;
-
     float2 q[kPer];
-    spread_and_transform<2>(sm, tw, t, y, n, fc, p.df, full);
+    spread_and_transform<2>(sm, tw, t, y, n, fc, p.df, 1.0f, s_sum);
 #pragma unroll
     for (int i = 0; i < kPer; i++) q[i] = mode(sm, tw, threadIdx.x + i * kThreads);
     __syncthreads();
-    spread_and_transform<1>(sm, tw, t, y, n, fc, p.df, y_scale);
+    spread_and_transform<1>(sm, tw, t, y, n, fc, p.df, y_max, s_sum);
 
     unsigned again = 0;  // the thread's near-singular modes
 #pragma unroll
@@ -300,9 +326,8 @@ __global__ void __launch_bounds__(kThreads, 2)
         if (k >= p.n_freq) continue;
         const float dc = deconv[kappa < 0 ? -kappa : kappa];
         const float2 sv = mode(sm, tw, j);
-        const float dy = dc * y_unit, dq = dc * q_unit;
-        const LSAcc a{sv.x * dy, sv.y * dy, 0.5f * fmaf(q[i].x, dq, (float)n),
-                      0.5f * q[i].y * dq};
+        const LSAcc a{sv.x * dc, sv.y * dc, 0.5f * fmaf(q[i].x, dc, (float)n),
+                      0.5f * q[i].y * dc};
         const float det = a.cos_cos * ((float)n - a.cos_cos) - a.cos_sin * a.cos_sin;
         if (!(det > kNufftSingular * (float)n * (float)n)) again |= 1u << i;
         out[k] = ls_power(a, n);

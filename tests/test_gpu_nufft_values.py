@@ -78,3 +78,51 @@ def test_values_that_are_not_finite(bad):
 
     # (4 times leaves room for clocks and launch gaps; the fault was 34 times.)
     assert best(spoilt) <= 4.0 * best(ms)
+
+
+def _power64(t, y, freqs):
+    import torch
+
+    t, y, f = (torch.from_numpy(np.asarray(x, np.float64)).cuda() for x in (t, y, freqs))
+    out = []
+    for fb in torch.split(f, max(1, 20_000_000 // len(t))):
+        th = t[:, None] * fb[None, :]
+        th = 2.0 * np.pi * (th - torch.round(th))
+        c, s = torch.cos(th), torch.sin(th)
+        C, S, cc, cs = y @ c, y @ s, (c * c).sum(0), (c * s).sum(0)
+        ss = len(t) - cc
+        out.append(0.5 * (ss * C * C - 2.0 * cs * C * S + cc * S * S) / (cc * ss - cs * cs))
+    return torch.cat(out).cpu().numpy()
+
+
+@pytest.mark.parametrize("n", [300, 511, 1023, 2000, 16384])
+@pytest.mark.parametrize("kind", ["one", "huge", "percent", "tails", "eclipses"])
+def test_values_far_from_the_rest(kind, n):
+    """A sinusoid with one value far off (as a leaked sentinel), one of 10^4,
+    one in a hundred far off, heavy tails, and eclipses.  Largest error 2e-5 of
+    the curve's peak, the bound of tests/test_gpu_nufft.py, and the error
+    (2-norm) no larger than the sincos form's; a quarter is left for the
+    spread of the two forms' rounding, of about n values each."""
+    rng = np.random.default_rng(n)
+    t = lc.seasonal_times(rng, n, 3000.0).astype(np.float32)
+    y = 0.3 * np.sin(2 * np.pi * 1.37 * t) + rng.normal(0, 0.05, n)
+    if kind == "one":
+        y[n // 3] = 85.0
+    elif kind == "huge":
+        y[n // 3] = -1e4
+    elif kind == "percent":
+        y[rng.integers(0, n, n // 100)] += 30.0
+        y[n // 2] = 85.0
+    elif kind == "tails":
+        y += 0.3 * rng.standard_t(1.5, n)
+    else:
+        y = np.where(np.mod(1.37 * t, 1.0) < 0.05, -0.5, 0.0) + rng.normal(0, 0.02, n)
+    y = (y - y.mean()).astype(np.float32)
+    f0, df, n_freq = 0.01, 0.002, 10000
+    want = _power64(t, y, f0 + df * np.arange(n_freq))
+    err = {form: _power([t], [y], f0, df, n_freq, form)[0] - want
+           for form in ("transform", "sincos")}
+    np.testing.assert_array_equal(_power([t], [y], f0, df, n_freq, "transform")[0],
+                                  _power([t], [y], f0, df, n_freq, "transform")[0])
+    assert np.abs(err["transform"]).max() <= 2e-5 * want.max()
+    assert np.linalg.norm(err["transform"]) <= 1.25 * np.linalg.norm(err["sincos"])
