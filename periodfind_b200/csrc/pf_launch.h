@@ -8,6 +8,28 @@
 
 namespace pfk {
 
+// Lets kernel k take `smem` bytes of dynamic shared memory.  The limit belongs
+// to the kernel on the device, not to a launch, and contexts launch from
+// several threads: it is only ever raised, to all that the kernel's static
+// memory leaves, as a limit of one call's size could be lowered by another
+// thread between its setting and the launch.
+template <class K>
+inline cudaError_t allow_smem(K k, size_t smem) {
+    if (smem <= 32u * 1024u) return cudaSuccess;  // within the default of 48 KB in all
+    cudaFuncAttributes a;
+    cudaError_t e = cudaFuncGetAttributes(&a, k);
+    if (e != cudaSuccess) return e;
+    if ((size_t)a.maxDynamicSharedSizeBytes >= smem) return cudaSuccess;
+    int dev = 0, optin = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) !=
+        cudaSuccess)
+        return e;
+    const size_t most = (size_t)optin - a.sharedSizeBytes;
+    if (smem > most) return cudaErrorInvalidValue;
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
 // KIND_LSREC: Lomb-Scargle on a uniform frequency grid with the
 // angle-addition recurrence along the grid (pf_lsrec.cuh); `rounds` holds
 // its frequencies per thread.

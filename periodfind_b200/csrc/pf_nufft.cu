@@ -401,8 +401,7 @@ cudaError_t launch_nufft_table(float* table, cudaStream_t s) {
 cudaError_t launch_nufft(const NufftParams& p, uint32_t n_curves, cudaStream_t s) {
     if (n_curves == 0) return cudaSuccess;
     const int smem = (int)sizeof(PF_KNS::Smem);
-    cudaError_t e = cudaFuncSetAttribute(PF_KNS::nufft_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = allow_smem(PF_KNS::nufft_kernel, smem);
     if (e != cudaSuccess) return e;
     PF_KNS::nufft_kernel<<<n_curves * p.blocks, PF_KNS::kThreads, smem, s>>>(p);
     return cudaGetLastError();

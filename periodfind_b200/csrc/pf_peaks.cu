@@ -537,8 +537,7 @@ cudaError_t launch_peaks(const float* pg, uint64_t n_curves, uint64_t flat_len,
     }
     const size_t smem = (size_t)kChunk * 12 + (size_t)n_peaks * 12;
     if (smem > 227u * 1024u) return cudaErrorInvalidValue;  // n_peaks > ~18000
-    cudaError_t e = cudaFuncSetAttribute(peaks_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(peaks_kernel, smem);
     if (e != cudaSuccess) return e;
     peaks_kernel<<<(unsigned)n_curves, kPeakThreads, smem, stream>>>(
         pg, flat_len, n_peaks, min_distance, use_max, out_idx, out_val);

@@ -452,8 +452,7 @@ cudaError_t launch_stats(const float* pg, uint64_t n_curves, uint32_t n_cells, i
     const int staged = with_row <= kStageBytes;
     if (staged) smem = with_row;
     if (smem > kStageBytes) return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(stats_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(stats_kernel, smem);
     if (e != cudaSuccess) return e;
     stats_kernel<<<(unsigned)n_curves, kStatThreads, smem, s>>>(
         pg, n_cells, use_max, n_top, depth, staged, stats, top_idx, top_val);
@@ -467,8 +466,7 @@ cudaError_t launch_prep_mags(const float* m, const int64_t* d_off, uint64_t n_cu
     if (n_curves > 0x7FFFFFFFull) return cudaErrorInvalidValue;
     const size_t smem = kind == 1 ? (size_t)4 << tree_depth(max_len) : 0;
     if (smem > 200u * 1024u) return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(prep_mags_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(prep_mags_kernel, smem);
     if (e != cudaSuccess) return e;
     prep_mags_kernel<<<(unsigned)n_curves, kPrepThreads, smem, s>>>(m, d_off, kind, out);
     return cudaGetLastError();
