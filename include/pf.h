@@ -489,7 +489,7 @@ int pf_center_mags(const float* const* mags, const uint64_t* lengths, uint64_t n
                    float* const* out);
 
 /* The autotuner's decisions on this context, one line per (computation,
- * length class): the launch shape kept and the sample times of the fastest
+ * load of the chip, length class): the launch shape kept and the sample times of the fastest
  * and slowest candidates.  Writes at most len bytes (NUL-terminated) and
  * returns the number of entries. */
 int pf_tuning_report(const pf_ctx* ctx, char* buf, uint64_t len);
