@@ -1155,7 +1155,8 @@ int launch_classes(pf_ctx* ctx, const Job& j, const Layout& L, const FoldConfig&
     if (j.mode & PF_ONE_LAUNCH) {
         // Every curve in one launch with the shape tuned for the class that
         // holds the most points (or, where that shape is the shared-histogram
-        // binning and longer curves are present, the longest class's).
+        // binning and longer curves are present, the longest class's; where
+        // it is the transform and there are curves too short for it, theirs).
         int d = -1, longest = -1;
         for (int c = 0; c < kClasses; c++) {
             if (!r[c].n) continue;
@@ -1163,6 +1164,9 @@ int launch_classes(pf_ctx* ctx, const Job& j, const Layout& L, const FoldConfig&
             longest = c;
         }
         if (cc[d].kind == KIND_BINWARP && longest > kWarpClassMax) d = longest;
+        if (cc[d].kind == KIND_NUFFT && !(j.mode & PF_TRIG_TRANSFORM))
+            for (int c = 0; c < kNufftClassMin; c++)
+                if (r[c].n) d = c;
         const FoldConfig one = cc[d];
         const uint64_t pts = L.total_pts;
         for (int c = 0; c < kClasses; c++) r[c] = Range{0, 0, 0};

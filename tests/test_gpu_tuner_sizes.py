@@ -58,3 +58,23 @@ def test_short_and_long_frequency_grids(monkeypatch):
         seen |= keys
     for order in ((1100, 15000), (15000, 1100)):
         assert len(_keys(monkeypatch, [call(n) for n in order])) == 2
+
+
+def test_one_launch_with_curves_too_short_for_the_transform(monkeypatch):
+    """PF_ONE_LAUNCH with curves under 64 points beside long ones: the short ones
+    keep the direct form that they have in a launch of their own."""
+    from periodfind_b200 import _native as nat
+    from periodfind_b200 import gpu
+
+    ctx = nat.Context(0)
+    monkeypatch.setattr(nat, "default_context", lambda device=0: ctx)
+    rng = np.random.default_rng(3)
+    lengths = [20, 33, 63] + [3000] * 8
+    ts = [lc.seasonal_times(rng, n, 3000.0).astype(np.float32) for n in lengths]
+    ms = [rng.normal(0, 1, n).astype(np.float32) for n in lengths]
+    grid = (0.01, 0.0004, 50000)
+    ls, one = gpu.LombScargle(), gpu.LombScargle()
+    one._flags |= nat.PF_ONE_LAUNCH
+    own = ls.periodograms_frequency_grid(ts, ms, *grid)
+    assert "trig=transform" in ctx.tuning_report()
+    np.testing.assert_array_equal(one.periodograms_frequency_grid(ts, ms, *grid)[:3], own[:3])
