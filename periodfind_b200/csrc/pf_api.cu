@@ -220,6 +220,7 @@ struct pf_ctx {
         bool persist;
         int rounds;
         int cells;
+        bool mixed;
         float ms;        // sample time of the winner
         float ms_worst;  // and of the slowest candidate
         uint32_t candidates;
@@ -603,6 +604,7 @@ int warps_per_sm(size_t smem, int block) {
 // size that gives the most resident warps for this histogram size.
 FoldConfig choose_config(pf_ctx* ctx, const Job& j, uint32_t max_len, bool& ok) {
     FoldConfig c{};
+    c.mixed = false;
     c.kind = KIND_FOLD;
     c.cnt16 = false;
     c.algo = j.algo;
@@ -922,7 +924,7 @@ cudaError_t launch_fold_sem(const Job& j, const FoldConfig& c, const FoldParams&
 // Launch shape of one length class.  Cached per context; the first time a
 // key is met, every candidate (the bin kernel: block 32 / 64 / 128 where
 // shared memory allows, 1 or 2 periods per thread at once (AOV also 3 at block
-// 64), in 1 or 4 rounds;
+// 64), in 1 or 4 rounds, for CE also with the points in their own order;
 // the others: block 64 / 128 / 256, persistent or one CTA per item) is timed
 // with CUDA events on a
 // sample of the class (a contiguous run of its curves from the middle of
@@ -959,6 +961,13 @@ int tuned_config(pf_ctx* ctx, const Job& j, const FoldConfig& base, int cls, uin
         out.persist = false;
         return PF_OK;
     }
+    // CE points in their own order: a candidate while a curve has few points
+    // for each column (the column sort won from 10-24 points a column on, later
+    // with larger histograms), and the base shape's form below 8.
+    const double per_column = (double)cls_points / (double)nc / (double)std::max(j.n_mag, 1u);
+    const bool mixed_ok = base.kind == KIND_BIN && base.algo == ALGO_CE && !base.ref_stats &&
+                          per_column < 24.0;
+    out.mixed = mixed_ok && per_column < 8.0;
     if (only_warp) {
         out.kind = KIND_BINWARP;
         out.block = 256;
@@ -973,6 +982,7 @@ int tuned_config(pf_ctx* ctx, const Job& j, const FoldConfig& base, int cls, uin
         out.persist = it->second.persist;
         out.rounds = it->second.rounds;
         out.cells = it->second.cells;
+        out.mixed = it->second.mixed;
         return true;
     };
     const int load = load_class(ctx, nc * j.n_per * j.n_pdt);
@@ -1003,7 +1013,8 @@ int tuned_config(pf_ctx* ctx, const Job& j, const FoldConfig& base, int cls, uin
     ps.bins = nullptr;
     ps.q.order = p.q.order + s0;
     ps.q.next = reinterpret_cast<unsigned*>((char*)ctx->d_misc.p + kCounterOffset) + kTuneCounter;
-    pf_ctx::Tuned best{out.kind, out.block, out.persist, out.rounds, out.cells, 1e30f, 0.0f, 0};
+    pf_ctx::Tuned best{out.kind,  out.block, out.persist, out.rounds,
+                       out.cells, out.mixed, 1e30f,       0.0f, 0};
     // Candidates: see above; for the recurrence 4 or 8 frequencies per
     // thread.  The reference statistic is built in one shape only.
     std::vector<FoldConfig> cands;
@@ -1023,7 +1034,10 @@ int tuned_config(pf_ctx* ctx, const Job& j, const FoldConfig& base, int cls, uin
                 for (int alt = 0; alt < (shapes ? 2 : 1); alt++) {
                     t.rounds = bin && alt ? 4 : 1;
                     t.persist = !bin && alt;
-                    cands.push_back(t);
+                    for (int own = 0; own < (mixed_ok && block <= 64 ? 2 : 1); own++) {
+                        t.mixed = own != 0;
+                        cands.push_back(t);
+                    }
                 }
             }
         }
@@ -1113,6 +1127,7 @@ int tuned_config(pf_ctx* ctx, const Job& j, const FoldConfig& base, int cls, uin
             best.persist = c.first.persist;
             best.rounds = c.first.rounds;
             best.cells = c.first.cells;
+            best.mixed = c.first.mixed;
         }
     }
     ctx->tuned[key] = best;
@@ -1121,6 +1136,7 @@ int tuned_config(pf_ctx* ctx, const Job& j, const FoldConfig& base, int cls, uin
     out.persist = best.persist;
     out.rounds = best.rounds;
     out.cells = best.cells;
+    out.mixed = best.mixed;
     return PF_OK;
 }
 
@@ -1260,19 +1276,22 @@ int device_pipeline(pf_ctx* ctx, const Job& j, const Layout& L, const FoldConfig
             n_runs = L.total_pts + 4 * (size_t)ncur;
         }
         const size_t o_runs = align_up(n_ts * 4 + 32, 256);
-        if ((rc = ensure_dev(ctx, ctx->d_aux32, o_runs + n_runs * 4)) != PF_OK) return rc;
+        const size_t o_cols = align_up(o_runs + n_runs * 4, 256);
+        if ((rc = ensure_dev(ctx, ctx->d_aux32, o_cols + L.total_pts * 2)) != PF_OK) return rc;
         float* ts = (float*)ctx->d_aux32.p;
         uint32_t* runs = (uint32_t*)((char*)ctx->d_aux32.p + o_runs);
+        uint16_t* cols = (uint16_t*)((char*)ctx->d_aux32.p + o_cols);
         p.ts = ts;
         p.runs = runs;
+        p.cols = cols;
         p.ts_mul = lay.ts_mul;
         p.ts_pad = lay.ts_pad;
         p.run_mul = lay.run_mul;
         p.run_pad = lay.run_pad;
         PF_CUDA(cpu ? launch_cesort_cpusem(p.t, p.m, dcurves, ncur, j.n_mag, p.mag_bin_size, lay,
-                                           ts, runs, s)
+                                           ts, runs, cols, s)
                     : launch_cesort_cudasem(p.t, p.m, dcurves, ncur, j.n_mag, p.mag_bin_size,
-                                            lay, ts, runs, s),
+                                            lay, ts, runs, cols, s),
                 "CE sort kernel");
         ctx->launches++;
         if (j.mode & PF_BINS_SHARED) {
@@ -2048,7 +2067,7 @@ int pf_tuning_report(const pf_ctx* ctx, char* buf, uint64_t len) {
     for (const auto& kv : ctx->tuned) {
         char line[320];
         snprintf(line, sizeof(line),
-                 "%s: %sblock=%d rounds=%d cells=%d %s sample_ms=%.3f slowest_ms=%.3f candidates=%u\n",
+                 "%s: %s%sblock=%d rounds=%d cells=%d %s sample_ms=%.3f slowest_ms=%.3f candidates=%u\n",
                  kv.first.c_str(),
                  kv.second.kind == KIND_LSREC ? "trig=recurrence "
                  : kv.second.kind == KIND_NUFFT ? "trig=transform "
@@ -2057,7 +2076,7 @@ int pf_tuning_report(const pf_ctx* ctx, char* buf, uint64_t len) {
                  : (kv.second.kind == KIND_FOLD && kv.first.find("fgrid") != std::string::npos)
                      ? "trig=sincos "
                      : "",
-                 kv.second.block, kv.second.rounds, std::max(kv.second.cells, 1),
+                 kv.second.mixed ? "points=own-order " : "", kv.second.block, kv.second.rounds, std::max(kv.second.cells, 1),
                  kv.second.persist ? "persistent" : "one-cta-per-item", kv.second.ms,
                  kv.second.ms_worst, kv.second.candidates);
         out += line;

@@ -41,7 +41,12 @@
 // reduction per evaluation were bound by the load.  Three things shrink it:
 //   - CE takes its points sorted by magnitude column (ce_sort_kernel), so a
 //     point is its time alone and the counter word and increment stay in
-//     registers for a column's run;
+//     registers for a column's run.  Curves with few points for each column
+//     they meet spend more on their runs (each padded to four points, about
+//     30 instructions) than that saves: MIXED takes the points in their own
+//     order with the column in the last bits of the time, five instructions
+//     more per point (10 x 40 columns, 120 points a curve: 1.05 -> 0.91 ms;
+//     10 x 64, 700 points: 0.94 -> 0.73).  The tuner weighs the two;
 //   - a thread holds CELLS = 2 periods, for AOV also 3, so one load serves as
 //     many evaluations (AOV samples from 256 points on 0.64 -> 0.60 ms with 3;
 //     CE 10% slower with 3, both slower with 4: too few warps); staging the
@@ -86,6 +91,20 @@ __device__ __forceinline__ void mul_wide_u32(uint32_t a, uint32_t b, uint32_t& l
     asm("{ .reg .u64 w; mul.wide.u32 w, %2, %3; mov.b64 {%0, %1}, w; }"
         : "=r"(lo), "=r"(hi)
         : "r"(a), "r"(b));
+}
+
+// A time that was a float has 29 zero bits at the end of its double; a CE
+// point's magnitude column (below 4096) is kept in the last 12.
+constexpr uint32_t kColumnBits = 0xFFFu;
+__device__ __forceinline__ double with_column(double t, uint32_t col) {
+    return __hiloint2double(__double2hiint(t), (int)((uint32_t)__double2loint(t) | col));
+}
+__device__ __forceinline__ uint32_t column_of(double t) {
+    return (uint32_t)__double2loint(t) & kColumnBits;
+}
+__device__ __forceinline__ double without_column(double t) {
+    return __hiloint2double(__double2hiint(t),
+                            (int)((uint32_t)__double2loint(t) & ~kColumnBits));
 }
 
 __device__ __forceinline__ void compiler_fence() { asm volatile("" ::: "memory"); }
@@ -151,7 +170,9 @@ __device__ __forceinline__ float aov_finish(double sbx, double xx_n, double sumx
 // the relative error near 1e-7 (FP64 here costs registers in the binning
 // loop, measured slower).  Per row, the magnitude bins are taken in pairs
 // (the two 16-bit halves of a word).  A cell's sum is one long chain of
-// loads, logs and adds, so two rows of every cell run side by side (tuning
+// loads, logs and adds, so two rows of every cell run side by side, with one
+// cell per thread (large histograms, few resident warps) four words of each
+// (10 x 64 columns, 20 points a curve: 2.51 -> 1.95 ms) (tuning
 // samples of 10 x 10 bins, one cell and row at a time -> this: [64,256) 1.31
 // -> 1.15 ms, [256,1024) 0.76 -> 0.70, [1024,4096) 0.60 -> 0.57; the floor is
 // the log's 110 operations per cell on the XU pipe).  8-bit counters for
@@ -170,7 +191,7 @@ __device__ __forceinline__ float lds_f32(uint32_t addr) {
     asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
     return v;
 }
-template <bool CNT16, int CELLS, bool TABLE>
+template <bool CNT16, int CELLS, bool TABLE, int UNROLL>
 __device__ __forceinline__ void ce_stat_fast(uint32_t tbase, uint32_t cell_bytes, uint32_t nP,
                                              uint32_t W, uint32_t cols, uint32_t n,
                                              uint32_t table, float (&out)[CELLS]) {
@@ -193,7 +214,7 @@ __device__ __forceinline__ void ce_stat_fast(uint32_t tbase, uint32_t cell_bytes
                 row[r][c] = 0.0f;
             }
         uint32_t at = tbase + j * (cols * 4u);
-#pragma unroll 1
+#pragma unroll UNROLL
         for (uint32_t wi = 0; wi < W; wi++, at += nP * (cols * 4u)) {
 #pragma unroll
             for (int r = 0; r < R; r++)
@@ -273,7 +294,8 @@ __device__ __forceinline__ void aov_sbx_fast(uint32_t tbase, uint32_t cell_bytes
 //         summed, with the 1/n scale taken out of the logs);
 //   AOV = (n - nP)/(nP - 1) * s1 / s2, s1 = sum_b X_b^2 / c_b - X^2 / n,
 //         s2 = sum x^2 - sum_b X_b^2 / c_b (X_b the fixed-point bin sums).
-template <int ALGO, bool CNT16, int BLOCK, bool REF_STATS, int ROUNDS, int CELLS>
+// MIXED (CE): points in their own order instead of sorted by column.
+template <int ALGO, bool CNT16, int BLOCK, bool REF_STATS, int ROUNDS, int CELLS, bool MIXED>
 __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, uint32_t item) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr uint32_t kCols = BLOCK * CELLS;  // counter columns of the CTA
@@ -337,11 +359,12 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
     const uint32_t edge32_lim = p.edge32_lim;
 
     // CE: the curve's sorted times and its runs of equal magnitude column
-    // (see ce_sort_kernel).  n_pad counts the runs' padding.
+    // (see ce_sort_kernel), n_pad counting the runs' padding; mixed: its points
+    // in their own order, each with its column.
     const float* src_t = p.t + cd.off;
     const uint32_t* runs = nullptr;
     uint32_t n_pad = n;
-    if constexpr (ALGO == ALGO_CE) {
+    if constexpr (ALGO == ALGO_CE && !MIXED) {
         src_t = p.ts + (cd.off * p.ts_mul + (int64_t)w.curve * p.ts_pad);
         runs = p.runs + (cd.off * p.run_mul + (int64_t)w.curve * p.run_pad);
         n_pad = runs[0];
@@ -352,20 +375,33 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
         const uint32_t n4 = (cnt + 3) >> 2;
         for (uint32_t i4 = tid; i4 < n4; i4 += BLOCK) {
             float4 q = gt[i4];
-            if constexpr (ALGO == ALGO_AOV) {
-                uint4 a = reinterpret_cast<const uint4*>(p.aux32 + cd.off + base)[i4];
-                // The packed arrays end in zeros; a repeated time with
-                // magnitude 0 keeps the padding out of the edge test of t = 0.
+            // The packed arrays end in zeros; a repeated time keeps the padding
+            // out of the edge test of t = 0.
+            if constexpr (ALGO == ALGO_AOV || MIXED) {
                 if (4 * i4 + 3 >= cnt) {
                     const float last = src_t[base + cnt - 1];
-                    if (4 * i4 + 1 >= cnt) { q.y = last; a.y = 0u; }
-                    if (4 * i4 + 2 >= cnt) { q.z = last; a.z = 0u; }
-                    if (4 * i4 + 3 >= cnt) { q.w = last; a.w = 0u; }
+                    if (4 * i4 + 1 >= cnt) q.y = last;
+                    if (4 * i4 + 2 >= cnt) q.z = last;
+                    if (4 * i4 + 3 >= cnt) q.w = last;
                 }
+            }
+            if constexpr (ALGO == ALGO_AOV) {
+                uint4 a = reinterpret_cast<const uint4*>(p.aux32 + cd.off + base)[i4];
+                if (4 * i4 + 1 >= cnt) a.y = 0u;
+                if (4 * i4 + 2 >= cnt) a.z = 0u;
+                if (4 * i4 + 3 >= cnt) a.w = 0u;
                 reinterpret_cast<uint4*>(tile_a)[i4] = a;
             }
-            reinterpret_cast<double2*>(tile_t)[2 * i4] = make_double2(q.x, q.y);
-            reinterpret_cast<double2*>(tile_t)[2 * i4 + 1] = make_double2(q.z, q.w);
+            double td[4] = {q.x, q.y, q.z, q.w};
+            if constexpr (MIXED) {
+                const ushort4 k = reinterpret_cast<const ushort4*>(p.cols + cd.off + base)[i4];
+                td[0] = with_column(td[0], k.x);
+                td[1] = with_column(td[1], k.y);
+                td[2] = with_column(td[2], k.z);
+                td[3] = with_column(td[3], k.w);
+            }
+            reinterpret_cast<double2*>(tile_t)[2 * i4] = make_double2(td[0], td[1]);
+            reinterpret_cast<double2*>(tile_t)[2 * i4 + 1] = make_double2(td[2], td[3]);
         }
     };
     // CE statistic by table (ce_stat_fast) where the table fits the staged
@@ -404,7 +440,7 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
             reinterpret_cast<uint32_t*>(cnt_raw)[k * kCols + c * BLOCK + tid] = 0u;
 
     uint32_t run_no = 0, run_at = 0, run = 0;  // CE: run number, its first position, its word
-    if constexpr (ALGO == ALGO_CE) run = runs[1];
+    if constexpr (ALGO == ALGO_CE && !MIXED) run = runs[1];
 
     for (uint32_t base = 0; base < n_pad; base += kBinTile) {
         const uint32_t cnt = min(kBinTile, n_pad - base);
@@ -489,6 +525,13 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
             }
         };
 
+        // The first word (row 0, cell 0) and the increment of a CE column.
+        auto column_word = [&](uint32_t col) -> uint32_t {
+            return tbase + (CNT16 ? col >> 1 : col) * (nP * kCols * 4);
+        };
+        auto column_unit = [&](uint32_t col) -> uint32_t {
+            return (CNT16 && (col & 1u)) ? unit << 16 : unit;
+        };
         auto body = [&](auto has_pdt_tag, auto fast_tag, auto f32_tag) {
             constexpr bool FAST = decltype(fast_tag)::value;
             constexpr bool F32 = decltype(f32_tag)::value;
@@ -503,6 +546,8 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
             // real: no branch per point; a group whose smallest edge-test
             // value is below the limit is revisited and its near-edge
             // points are moved to the reference's bin.
+            // Mixed: each point's counter word and increment come from its
+            // column instead of from the run.
             auto group = [&](auto g_tag, auto mask_tag, uint32_t i, uint32_t live, uint32_t at,
                              uint32_t inc) {
                 constexpr int G = decltype(g_tag)::value;
@@ -530,13 +575,20 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
                 for (int c = 0; c < CELLS; c++) emin[c] = 0xFFFFFFFFu;
 #pragma unroll
                 for (int k = 0; k < G; k++) {
-                    const uint32_t ik = (!MASK || (uint32_t)k < live) ? inc : 0u;
+                    uint32_t ak = at, ik = inc;
+                    if constexpr (MIXED) {
+                        const uint32_t col = column_of(td[k]);
+                        ak = column_word(col);
+                        ik = column_unit(col);
+                        td[k] = without_column(td[k]);
+                    }
+                    if (MASK && (uint32_t)k >= live) ik = 0u;
 #pragma unroll
                     for (int c = 0; c < CELLS; c++) {
                         uint32_t ev;
                         const uint32_t row = bin_of(td[k], ys[c], pc[c], ev);
                         emin[c] = min(emin[c], ev);
-                        add(row, at + c * BLOCK * 4, ik, ALGO == ALGO_AOV ? ta[k] : 0u);
+                        add(row, ak + c * BLOCK * 4, ik, ALGO == ALGO_AOV ? ta[k] : 0u);
                     }
                 }
                 uint32_t em = emin[0];
@@ -569,7 +621,13 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
                         const uint32_t c = e / G, k = e % G;
                         Cell s;
                         cell_setup<FOLD_EXACT>(s, p.periods[cell_period(c)], period_dt);
-                        const double t = tile_t[i + k];
+                        double t = tile_t[i + k];
+                        uint32_t ak = at, ik = inc;
+                        if constexpr (MIXED) {
+                            ak = column_word(column_of(t));
+                            ik = column_unit(column_of(t));
+                            t = without_column(t);
+                        }
                         uint32_t ev;
                         const uint32_t row = bin_of(t, s.yhi * y_scale, s.c, ev);
                         const uint32_t ex =
@@ -577,8 +635,8 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
                         if (ex != row) {
                             // u32 wraparound keeps packed halves and sums exact.
                             const uint32_t a = ALGO == ALGO_AOV ? tile_a[i + k] : 0u;
-                            add(row, at + c * BLOCK * 4, 0u - inc, 0u - a);
-                            add(ex, at + c * BLOCK * 4, inc, a);
+                            add(row, ak + c * BLOCK * 4, 0u - ik, 0u - a);
+                            add(ex, ak + c * BLOCK * 4, ik, a);
                         }
                     }
                 }
@@ -586,7 +644,7 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
             // m points from tile position i (a multiple of 4).
             auto span = [&](uint32_t i, uint32_t m, uint32_t at, uint32_t inc) {
                 if constexpr (FAST) {
-                    // Groups of 16 (CE; 16 were slower for AOV, whose two
+                    // Groups of 16 (CE runs; 16 were slower for AOV, whose two
                     // reductions per point need the registers), then 8, 4
                     // and the rest of the last four.
                     using G16 = std::integral_constant<int, 16>;
@@ -594,7 +652,7 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
                     using G4 = std::integral_constant<int, 4>;
                     using Whole = std::false_type;
                     uint32_t k = 0;
-                    if constexpr (ALGO == ALGO_CE) {
+                    if constexpr (ALGO == ALGO_CE && !MIXED) {
 #pragma unroll 1
                         for (; k + 16 <= m; k += 16) group(G16{}, Whole{}, i + k, 16u, at, inc);
                         if (k + 8 <= m) {
@@ -616,14 +674,24 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
                         Cell s;
                         cell_setup<FOLD_EXACT>(s, p.periods[cell_period(c)], period_dt);
 #pragma unroll 2
-                        for (uint32_t k = 0; k < m; k++)
-                            add(exact_row(tile_t[i + k], s, has_pdt_tag), at + c * BLOCK * 4, inc,
+                        for (uint32_t k = 0; k < m; k++) {
+                            double t = tile_t[i + k];
+                            uint32_t ak = at, ik = inc;
+                            if constexpr (MIXED) {
+                                ak = column_word(column_of(t));
+                                ik = column_unit(column_of(t));
+                                t = without_column(t);
+                            }
+                            add(exact_row(t, s, has_pdt_tag), ak + c * BLOCK * 4, ik,
                                 ALGO == ALGO_AOV ? tile_a[i + k] : 0u);
+                        }
                     }
                 }
             };
             if constexpr (ALGO == ALGO_AOV) {
                 span(0u, cnt, tbase, 1u);
+            } else if constexpr (MIXED) {
+                span(0u, cnt, 0u, 0u);
             } else {
                 // The runs (one magnitude column each) that meet this tile.
                 const uint32_t end = base + cnt;
@@ -631,10 +699,8 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
                     const uint32_t len = run & 0xFFFFu, col = run >> 16;
                     const uint32_t lo = max(run_at, base), hi = min(run_at + len, end);
                     const uint32_t next = runs[run_no + 2];
-                    const uint32_t word = CNT16 ? col >> 1 : col;
                     if (hi > lo)
-                        span(lo - base, hi - lo, tbase + word * (nP * kCols * 4),
-                             (CNT16 && (col & 1u)) ? unit << 16 : unit);
+                        span(lo - base, hi - lo, column_word(col), column_unit(col));
                     const uint32_t next_at = run_at + ((len + 3u) & ~3u);
                     if (next_at > end) break;  // the rest lies in the next tile
                     run_at = next_at;
@@ -669,12 +735,14 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
         if (active) {
             float res[CELLS];
             if constexpr (ALGO == ALGO_CE) {
+                constexpr int kUnroll = CELLS == 1 ? 4 : MIXED ? 2 : 1;
                 if (table)
-                    ce_stat_fast<CNT16, CELLS, true>(
+                    ce_stat_fast<CNT16, CELLS, true, kUnroll>(
                         tbase, BLOCK * 4, nP, W, kCols, n,
                         (uint32_t)__cvta_generic_to_shared(tile_t), res);
                 else
-                    ce_stat_fast<CNT16, CELLS, false>(tbase, BLOCK * 4, nP, W, kCols, n, 0u, res);
+                    ce_stat_fast<CNT16, CELLS, false, kUnroll>(tbase, BLOCK * 4, nP, W, kCols, n,
+                                                               0u, res);
             } else {
                 double sbx[CELLS];
                 aov_sbx_fast<CELLS>(tbase, BLOCK * 4, nP, kCols, sbx);
@@ -766,10 +834,10 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
 // One CTA per item of the device work queue (see WorkQueue); an item is
 // ROUNDS x CELLS x BLOCK consecutive periods.  (Persistent CTAs measured 1-8%
 // slower in every class.)
-template <int ALGO, bool CNT16, int BLOCK, bool REF_STATS, int ROUNDS, int CELLS>
+template <int ALGO, bool CNT16, int BLOCK, bool REF_STATS, int ROUNDS, int CELLS, bool MIXED>
 __global__ void __launch_bounds__(BLOCK, bin_min_blocks<ALGO, BLOCK, CELLS>())
     bin_kernel(const FoldParams p) {
-    bin_item<ALGO, CNT16, BLOCK, REF_STATS, ROUNDS, CELLS>(
+    bin_item<ALGO, CNT16, BLOCK, REF_STATS, ROUNDS, CELLS, MIXED>(
         p, queue_item<BLOCK * ROUNDS * CELLS>(p, blockIdx.x), blockIdx.x);
 }
 
@@ -779,12 +847,13 @@ __global__ void __launch_bounds__(BLOCK, bin_min_blocks<ALGO, BLOCK, CELLS>())
 // instead of a 16-byte record).  Counts do not depend on the order.  Per
 // curve: ts = the runs one after the other, each padded to a multiple of 4
 // with repeats of its first time; runs = {padded total, then one word
-// (column << 16) | length per non-empty column, then 0}.
+// (column << 16) | length per non-empty column, then 0}.  cols = the column of
+// each point in the curve's own order, for the MIXED form.
 __global__ void __launch_bounds__(256)
     ce_sort_kernel(const float* __restrict__ t, const float* __restrict__ m,
                    const CurveDesc* __restrict__ curves, uint32_t n_curves, uint32_t n_mag,
                    float mag_bin_size, CeSortLayout lay, float* __restrict__ ts,
-                   uint32_t* __restrict__ runs) {
+                   uint32_t* __restrict__ runs, uint16_t* __restrict__ cols) {
     extern __shared__ uint32_t sort_cnt[];  // [n_mag] counts, [n_mag] write positions
     uint32_t* sort_pos = sort_cnt + n_mag;
     const uint32_t c = blockIdx.x;
@@ -800,7 +869,12 @@ __global__ void __launch_bounds__(256)
     };
     for (uint32_t k = threadIdx.x; k < n_mag; k += 256) sort_cnt[k] = 0u;
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < cd.n; i += 256) atomicAdd(&sort_cnt[column(i)], 1u);
+    for (uint32_t i = threadIdx.x; i < cd.n; i += 256) {
+        const uint32_t k = column(i);
+        cols[cd.off + i] = (uint16_t)k;
+        atomicAdd(&sort_cnt[k], 1u);
+    }
+    for (uint32_t i = cd.n + threadIdx.x; i < ((cd.n + 3u) & ~3u); i += 256) cols[cd.off + i] = 0;
     __syncthreads();
     if (threadIdx.x == 0) {
         uint32_t at = 0, r = 0;
@@ -815,7 +889,7 @@ __global__ void __launch_bounds__(256)
     }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < cd.n; i += 256)
-        tc[atomicAdd(&sort_pos[column(i)], 1u)] = t[cd.off + i];
+        tc[atomicAdd(&sort_pos[cols[cd.off + i]], 1u)] = t[cd.off + i];
     __syncthreads();
     for (uint32_t k = threadIdx.x; k < n_mag; k += 256) {
         const uint32_t len = sort_cnt[k], end = sort_pos[k];

@@ -59,7 +59,7 @@ struct FoldConfig {
     int algo;   // ALGO_*
     int fold;   // FOLD_*
     int acc;    // AOVACC_* (AOV only)
-    int block;  // threads per CTA: 64, 128 or 256
+    int block;  // threads per CTA: 64, 128 or 256; bin kernel 32, 64 or 128
     bool ovl;   // general bin-overlap path
     bool ref_stats; // bin_kernel: the reference's statistic operation sequence
     bool persist;   // queue kernels but the bin kernel: persistent grid instead of
@@ -67,6 +67,7 @@ struct FoldConfig {
     int rounds;     // bin kernel: an item is rounds x cells x block periods (1 or 4);
                     // KIND_LSREC: frequencies per thread (4 or 8)
     int cells;      // bin kernel: periods a thread holds at once (1, 2 or, AOV, 3)
+    bool mixed;     // CE bin kernel: points in their own order (block 32 and 64)
     int n_sm;       // persistent kernels: grid = n_sm x resident CTAs per SM
 };
 
@@ -100,14 +101,14 @@ cudaError_t launch_binaux_cudasem(const float* m, void* aux, const CurveDesc* cu
 cudaError_t launch_cesort_cudasem(const float* t, const float* m, const CurveDesc* curves,
                                   uint32_t n_curves, uint32_t n_mag, float mag_bin_size,
                                   const CeSortLayout& lay, float* ts, uint32_t* runs,
-                                  cudaStream_t s);
+                                  uint16_t* cols, cudaStream_t s);
 cudaError_t launch_binaux_cpusem(const float* m, void* aux, const CurveDesc* curves,
                                   uint32_t n_curves, uint32_t n_mag, float mag_bin_size,
                                   cudaStream_t s);
 cudaError_t launch_cesort_cpusem(const float* t, const float* m, const CurveDesc* curves,
                                   uint32_t n_curves, uint32_t n_mag, float mag_bin_size,
                                   const CeSortLayout& lay, float* ts, uint32_t* runs,
-                                  cudaStream_t s);
+                                  uint16_t* cols, cudaStream_t s);
 
 // FPW and BLS (pf_fpw.cuh): per point t, inverse variance iv = 1 / err^2 and
 // ivy = iv * m, packed per curve at off[c] with len[c] points; out is

@@ -73,6 +73,7 @@ struct FoldParams {
     const uint64_t* aux64;   // AOV FIX: packed (1 << 44) + fixed-point mag
     const float* ts;         // CE bin kernel: times sorted by magnitude column
     const uint32_t* runs;    // CE bin kernel: the columns' runs
+    const uint16_t* cols;    // CE bin kernel: each point's column, in the curves' own order
     uint32_t ts_mul, ts_pad, run_mul, run_pad;  // their CeSortLayout
     const CurveDesc* curves;
     const WorkItem* work;
