@@ -921,6 +921,15 @@ cudaError_t launch_fold_sem(const Job& j, const FoldConfig& c, const FoldParams&
                                      : launch_fold_cudasem(c, p, n_work, s);
 }
 
+// May a call use the shared-histogram binning?  With PF_BINS_SHARED, and where
+// 64 private histograms leave no room for a second CTA on the SM: 50 x 20 bins
+// on curves of 700 points 1.03 ms against 1.30 privatised.  With smaller ones
+// its samples were 1.3-5x the privatised form's in every class.
+bool bins_shared(const Job& j) {
+    return (j.mode & PF_BINS_SHARED) ||
+           bin_smem_bytes(j.algo, j.algo == ALGO_CE, 64, j.n_phase, j.n_mag) > 96u * 1024u;
+}
+
 // Launch shape of one length class.  Cached per context; the first time a
 // key is met, every candidate (the bin kernel: block 32 / 64 / 128 where
 // shared memory allows, 1 or 2 periods per thread at once (AOV also 3 at block
@@ -945,11 +954,10 @@ int tuned_config(pf_ctx* ctx, const Job& j, const FoldConfig& base, int cls, uin
     const bool only_fft = rec_ok && !only_rec && (j.mode & PF_TRIG_TRANSFORM);
     const bool no_rec = !rec_ok || only_fft || (j.mode & PF_TRIG_SINCOS);
     // PF_BINS_SHARED takes the shared-histogram binning where the curves fit
-    // it.  It is no candidate otherwise: its samples were 1.3-5x the
-    // privatised form's on every class measured, before that form's newer
-    // shapes.
-    const bool only_warp = base.kind == KIND_BIN && !base.ref_stats && cls <= kWarpClassMax &&
-                           (j.mode & PF_BINS_SHARED);
+    // it.  Otherwise it is a candidate for large histograms (bins_shared).
+    const bool warp_ok = base.kind == KIND_BIN && !base.ref_stats && cls <= kWarpClassMax &&
+                         bins_shared(j);
+    const bool only_warp = warp_ok && (j.mode & PF_BINS_SHARED);
     if (only_rec) {
         out.kind = KIND_LSREC;
         out.block = 256;
@@ -1043,7 +1051,7 @@ int tuned_config(pf_ctx* ctx, const Job& j, const FoldConfig& base, int cls, uin
         }
     }
     // The shared-histogram binning (one histogram per warp and period).
-    if (only_warp) {
+    if (warp_ok) {
         for (int block : {128, 256})
             for (int persist = 0; persist < 2; persist++) {
                 FoldConfig t = base;
@@ -1294,7 +1302,7 @@ int device_pipeline(pf_ctx* ctx, const Job& j, const Layout& L, const FoldConfig
                                             lay, ts, runs, cols, s),
                 "CE sort kernel");
         ctx->launches++;
-        if (j.mode & PF_BINS_SHARED) {
+        if (bins_shared(j)) {
             if ((rc = ensure_dev(ctx, ctx->d_aux64, L.total_pts * 8 + 32)) != PF_OK) return rc;
             p.aux64 = (const uint64_t*)ctx->d_aux64.p;
             PF_CUDA(cpu ? launch_binaux_cpusem(p.m, ctx->d_aux64.p, dcurves, ncur, j.n_mag,

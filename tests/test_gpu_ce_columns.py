@@ -33,3 +33,31 @@ def test_time_of_many_columns():
     same points.  Sorted by column alone the call took 4 times as long; with
     the points in their own order it takes 2.2 times."""
     assert _device_ms(10, 40, 60) <= 3.0 * _device_ms(10, 10, 60)
+
+
+@pytest.mark.parametrize("shared", [False, True])
+def test_large_histograms_may_share_them(monkeypatch, shared):
+    """Where 64 private histograms fill an SM, the tuner weighs one histogram
+    per warp and period as well; with small ones it does
+    not.  The values are the same bit for bit."""
+    from periodfind_b200 import _native as nat
+    from periodfind_b200 import gpu
+
+    ctx = nat.Context(0)
+    monkeypatch.setattr(nat, "default_context", lambda device=0: ctx)
+    rng = np.random.default_rng(2)
+    ts = [np.sort(rng.uniform(0, 900, n)).astype(np.float32) for n in (300, 700) for _ in range(30)]
+    ms = [rng.uniform(0.01, 0.99, len(t)).astype(np.float32) for t in ts]
+    periods = np.geomspace(0.1, 30.0, 1000).astype(np.float32)
+    bins = (50, 20) if shared else (10, 20)
+    ce, alone = gpu.ConditionalEntropy(*bins), gpu.ConditionalEntropy(*bins)
+    got = ce.periodograms(ts, ms, periods, np.zeros(1, np.float32))
+    report = ctx.tuning_report()
+    # Private histograms: 3 shapes of 50 x 20 bins fit, all 6 of 10 x 20, in 1
+    # or 4 rounds; shared ones: 2 shapes, persistent or not.
+    assert f"candidates={3 * 2 + 4 if shared else 6 * 2}" in report, report
+    other = nat.Context(0)
+    monkeypatch.setattr(nat, "default_context", lambda device=0: other)
+    alone._flags |= nat.PF_NO_TUNE
+    np.testing.assert_array_equal(
+        got, alone.periodograms(ts, ms, periods, np.zeros(1, np.float32)))
