@@ -512,10 +512,11 @@ cudaError_t launch_peaks(const float* pg, uint64_t n_curves, uint64_t flat_len,
     if (n_peaks <= 32) {
         // Parts per row: while there are at most eight warps per SM (740 rows
         // in eight parts were slower than one warp per row, 192 against 155
-        // us), at least two steps of samples each.
+        // us), rows of at least 16 steps of samples (shorter ones took 5 to 8 us
+        // longer split than with one warp), four or more for each part.
         int seg = 1;
         while (min_distance <= 1 && seg < kSplitWarps && n_curves * seg * 2 <= 148 * 8 &&
-               flat_len >= (uint64_t)seg * 4 * kWarpStep)
+               flat_len >= (uint64_t)(seg > 2 ? seg * 8 : 16) * kWarpStep)
             seg *= 2;
         if (seg > 1) {
             const unsigned rows = kSplitWarps / seg;
