@@ -350,7 +350,9 @@ __global__ void __launch_bounds__(kLsThreads, 2)
     const uint32_t ntiles = (n + kLsTile - 1) / kLsTile;
 
     for (uint32_t j = 0; j < rounds; j++) {
-        const uint64_t k0 = ((uint64_t)g * rounds + j) * (kLsWarps * kMulti) + wid * kMulti;
+        const uint64_t set = ((uint64_t)g * rounds + j) * (kLsWarps * kMulti);
+        if (set >= p.n_freq) break;  // uniform over the CTA: no frequency is left
+        const uint64_t k0 = set + wid * kMulti;
         double f[kMulti];
         F2 fp[kMulti];
         bool df[kMulti], all_df = true;  // uniform per warp
