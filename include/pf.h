@@ -494,6 +494,19 @@ int pf_center_mags(const float* const* mags, const uint64_t* lengths, uint64_t n
  * returns the number of entries. */
 int pf_tuning_report(const pf_ctx* ctx, char* buf, uint64_t len);
 
+/* Pin the launch shape of the chosen CE / AOV bin kernel on this context
+ * instead of tuning it: threads per CTA (32, 64 or 128), trial periods per
+ * thread (1, 2 or, AOV with 64 threads, 3), rounds per CTA (1 or 4) and, for
+ * CE with 32 or 64 threads, the points in their own order (1) or sorted by
+ * magnitude column (0).  A block of 0 returns to the tuner.  Values do not
+ * depend on the shape.  Calls whose histogram does not fit the shape are
+ * PF_EUNSUPPORTED. */
+int pf_pin_bin_shape(pf_ctx* ctx, int block, int cells, int rounds, int own_order);
+
+/* The bin kernel's reciprocals of the counts 1 .. n (n < 65536) on the device,
+ * in the arithmetic of `mode`'s semantics. */
+int pf_count_rcp_dev(pf_ctx* ctx, int mode, uint32_t n, double* d_out, void* stream);
+
 /* Number of kernels this context has launched since creation (telemetry
  * for benchmarks: launches of the library's own kernels only). */
 uint64_t pf_launch_count(const pf_ctx* ctx);

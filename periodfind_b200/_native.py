@@ -104,6 +104,8 @@ SIGNATURES = {
                             _vp], _int),
     "pf_ls_refine_dev": ([_vp, _vp, _vp, _vp, _u64, _vp, _vp, _u64, _u32, _vp, _vp, _vp], _int),
     "pf_tuning_report": ([_vp, ctypes.c_char_p, _u64], _int),
+    "pf_pin_bin_shape": ([_vp, _int, _int, _int, _int], _int),
+    "pf_count_rcp_dev": ([_vp, _int, _u32, _vp, _vp], _int),
     "pf_normalize_mags": ([_vp, _vp, _u64, _vp], _int),
     "pf_center_mags": ([_vp, _vp, _u64, _vp], _int),
     "pf_plan_create": ([_int, _int, _vp, _vp, _vp, _u64, _vp, _u64, _vp, _u64, _u32, _u32, _u32,

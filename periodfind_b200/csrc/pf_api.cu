@@ -226,6 +226,11 @@ struct pf_ctx {
         uint32_t candidates;
     };
     std::map<std::string, Tuned> tuned;
+    // pf_pin_bin_shape (block 0: none).
+    struct {
+        int block = 0, cells = 1, rounds = 1;
+        bool mixed = false;
+    } pin;
     // PF_ASYNC peak calls not yet collected by pf_wait, oldest first.  Each
     // copies its peaks into its own pinned block; the event follows the copy.
     struct Pending {
@@ -981,6 +986,16 @@ int tuned_config(pf_ctx* ctx, const Job& j, const FoldConfig& base, int cls, uin
         out.block = 256;
         out.rounds = 1;
         out.persist = false;
+    }
+    if (ctx->pin.block && base.kind == KIND_BIN && !base.ref_stats && !only_warp) {
+        out.block = ctx->pin.block;
+        out.cells = ctx->pin.cells;
+        out.rounds = ctx->pin.rounds;
+        out.mixed = ctx->pin.mixed;
+        if ((out.mixed && base.algo != ALGO_CE) || (out.cells == 3 && base.algo != ALGO_AOV) ||
+            fold_smem(out, j.n_phase, j.n_mag) > ctx->smem_optin)
+            return fail(ctx, PF_EUNSUPPORTED, "the pinned launch shape does not fit this call");
+        return PF_OK;
     }
     auto kept = [&](const std::string& k) -> bool {
         auto it = ctx->tuned.find(k);
@@ -2066,6 +2081,35 @@ int pf_center_mags(const float* const* mags, const uint64_t* lengths, uint64_t n
     }
     auto one = [&](uint64_t c) { center_curve(mags[c], lengths[c], out[c]); };
     for_each_curve(n_curves, total, one);
+    return PF_OK;
+}
+
+int pf_pin_bin_shape(pf_ctx* ctx, int block, int cells, int rounds, int own_order) {
+    if (!ctx) return PF_EINVAL;
+    const bool ok = block == 0 ||
+                    ((block == 32 || block == 64 || block == 128) && cells >= 1 &&
+                     (cells <= 2 || (cells == 3 && block == 64)) && (rounds == 1 || rounds == 4) &&
+                     (!own_order || block <= 64));
+    if (!ok)
+        return fail(ctx, PF_EINVAL, "no launch shape of %d threads, %d periods, %d rounds", block,
+                    cells, rounds);
+    ctx->pin.block = block;
+    ctx->pin.cells = cells;
+    ctx->pin.rounds = rounds;
+    ctx->pin.mixed = own_order != 0;
+    return PF_OK;
+}
+
+int pf_count_rcp_dev(pf_ctx* ctx, int mode, uint32_t n, double* d_out, void* stream) {
+    if (!ctx) return PF_EINVAL;
+    if (n >= 65536u) return fail(ctx, PF_EINVAL, "counts are below 65536, got %u", n);
+    if (n == 0) return PF_OK;
+    if (!d_out) return fail(ctx, PF_EINVAL, "NULL pointer argument");
+    PF_CUDA(cudaSetDevice(ctx->device), "cudaSetDevice");
+    PF_CUDA(use_cpu_semantics(mode) ? launch_count_rcp_cpusem(n, d_out, (cudaStream_t)stream)
+                                    : launch_count_rcp_cudasem(n, d_out, (cudaStream_t)stream),
+            "count reciprocal kernel");
+    ctx->launches++;
     return PF_OK;
 }
 

@@ -263,6 +263,11 @@ __device__ __forceinline__ double count_rcp(uint32_t c) {
     return __fma_rn(r, __fma_rn(-x, r, 1.0), r);
 }
 
+__global__ void count_rcp_kernel(uint32_t n, double* __restrict__ out) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = count_rcp(i + 1u);
+}
+
 // The chosen form's AOV sum_b X_b^2 / c_b over the fixed-point bin sums X_b
 // (empty bins have X_b = 0 and contribute nothing), CELLS cells at once
 // ([64,256) samples 0.87 -> 0.81 ms against library reciprocals and integer

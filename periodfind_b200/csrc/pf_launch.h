@@ -110,6 +110,10 @@ cudaError_t launch_cesort_cpusem(const float* t, const float* m, const CurveDesc
                                   const CeSortLayout& lay, float* ts, uint32_t* runs,
                                   uint16_t* cols, cudaStream_t s);
 
+// The bin kernel's reciprocals of the counts 1 .. n.
+cudaError_t launch_count_rcp_cudasem(uint32_t n, double* out, cudaStream_t s);
+cudaError_t launch_count_rcp_cpusem(uint32_t n, double* out, cudaStream_t s);
+
 // FPW and BLS (pf_fpw.cuh): per point t, inverse variance iv = 1 / err^2 and
 // ivy = iv * m, packed per curve at off[c] with len[c] points; out is
 // [curve][period][pdt].  bin_size = 1 / n_bins as the reference rounds it.
