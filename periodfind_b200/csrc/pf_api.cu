@@ -975,11 +975,14 @@ int tuned_config(pf_ctx* ctx, const Job& j, const FoldConfig& base, int cls, uin
         return PF_OK;
     }
     // CE points in their own order: a candidate while a curve has few points
-    // for each column (the column sort won from 10-24 points a column on, later
-    // with larger histograms), and the base shape's form below 8.
+    // for each column, fewer than there are columns (measured on 20 to 2000
+    // points: with 10 columns the column sort won from about 100 points on, with
+    // 20 from 300, with 40 from 1500, with 64 not up to 2000; the larger the
+    // histogram, the fewer the warps that hide a run's latency), and the base
+    // shape's form below 8.
     const double per_column = (double)cls_points / (double)nc / (double)std::max(j.n_mag, 1u);
     const bool mixed_ok = base.kind == KIND_BIN && base.algo == ALGO_CE && !base.ref_stats &&
-                          per_column < 24.0;
+                          per_column < (double)j.n_mag;
     out.mixed = mixed_ok && per_column < 8.0;
     if (only_warp) {
         out.kind = KIND_BINWARP;

@@ -380,33 +380,34 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
         const uint32_t n4 = (cnt + 3) >> 2;
         for (uint32_t i4 = tid; i4 < n4; i4 += BLOCK) {
             float4 q = gt[i4];
-            // The packed arrays end in zeros; a repeated time keeps the padding
-            // out of the edge test of t = 0.
-            if constexpr (ALGO == ALGO_AOV || MIXED) {
+            if constexpr (ALGO == ALGO_AOV) {
+                uint4 a = reinterpret_cast<const uint4*>(p.aux32 + cd.off + base)[i4];
+                // The packed arrays end in zeros; a repeated time with
+                // magnitude 0 keeps the padding out of the edge test of t = 0.
+                if (4 * i4 + 3 >= cnt) {
+                    const float last = src_t[base + cnt - 1];
+                    if (4 * i4 + 1 >= cnt) { q.y = last; a.y = 0u; }
+                    if (4 * i4 + 2 >= cnt) { q.z = last; a.z = 0u; }
+                    if (4 * i4 + 3 >= cnt) { q.w = last; a.w = 0u; }
+                }
+                reinterpret_cast<uint4*>(tile_a)[i4] = a;
+            }
+            if constexpr (MIXED) {
                 if (4 * i4 + 3 >= cnt) {
                     const float last = src_t[base + cnt - 1];
                     if (4 * i4 + 1 >= cnt) q.y = last;
                     if (4 * i4 + 2 >= cnt) q.z = last;
                     if (4 * i4 + 3 >= cnt) q.w = last;
                 }
-            }
-            if constexpr (ALGO == ALGO_AOV) {
-                uint4 a = reinterpret_cast<const uint4*>(p.aux32 + cd.off + base)[i4];
-                if (4 * i4 + 1 >= cnt) a.y = 0u;
-                if (4 * i4 + 2 >= cnt) a.z = 0u;
-                if (4 * i4 + 3 >= cnt) a.w = 0u;
-                reinterpret_cast<uint4*>(tile_a)[i4] = a;
-            }
-            double td[4] = {q.x, q.y, q.z, q.w};
-            if constexpr (MIXED) {
                 const ushort4 k = reinterpret_cast<const ushort4*>(p.cols + cd.off + base)[i4];
-                td[0] = with_column(td[0], k.x);
-                td[1] = with_column(td[1], k.y);
-                td[2] = with_column(td[2], k.z);
-                td[3] = with_column(td[3], k.w);
+                reinterpret_cast<double2*>(tile_t)[2 * i4] =
+                    make_double2(with_column(q.x, k.x), with_column(q.y, k.y));
+                reinterpret_cast<double2*>(tile_t)[2 * i4 + 1] =
+                    make_double2(with_column(q.z, k.z), with_column(q.w, k.w));
+            } else {
+                reinterpret_cast<double2*>(tile_t)[2 * i4] = make_double2(q.x, q.y);
+                reinterpret_cast<double2*>(tile_t)[2 * i4 + 1] = make_double2(q.z, q.w);
             }
-            reinterpret_cast<double2*>(tile_t)[2 * i4] = make_double2(td[0], td[1]);
-            reinterpret_cast<double2*>(tile_t)[2 * i4 + 1] = make_double2(td[2], td[3]);
         }
     };
     // CE statistic by table (ce_stat_fast) where the table fits the staged
