@@ -1117,17 +1117,39 @@ int tuned_config(pf_ctx* ctx, const Job& j, const FoldConfig& base, int cls, uin
     };
     // First pass: a warm-up launch, then the faster of two.
     std::vector<std::pair<FoldConfig, float>> timed;
-    for (const FoldConfig& t : cands) {
-        const uint64_t nw = queue_items(j, k, item_periods(t));
-        if (nw == 0 || nw > 0x7FFFFFFFull) continue;
-        float warm = 1e30f, ms = 1e30f;
-        int rc;
-        if ((rc = time_cand(t, 1, warm)) != PF_OK || (rc = time_cand(t, 2, ms)) != PF_OK)
-            return rc;
-        timed.emplace_back(t, ms);
-        best.candidates++;
-        best.ms_worst = std::max(best.ms_worst, ms);
-    }
+    auto time_all = [&](auto take) -> int {
+        for (const FoldConfig& t : cands) {
+            if (!take(t)) continue;
+            const uint64_t nw = queue_items(j, k, item_periods(t));
+            if (nw == 0 || nw > 0x7FFFFFFFull) continue;
+            float warm = 1e30f, ms = 1e30f;
+            int rc;
+            if ((rc = time_cand(t, 1, warm)) != PF_OK || (rc = time_cand(t, 2, ms)) != PF_OK)
+                return rc;
+            timed.emplace_back(t, ms);
+            best.candidates++;
+            best.ms_worst = std::max(best.ms_worst, ms);
+        }
+        return PF_OK;
+    };
+    // CE's two point orders are weighed with 1 and 2 periods per thread in the
+    // base shape's block, and the other shapes then timed for the faster order
+    // only: both in every shape made a plan of short curves 51 -> 68 ms to
+    // prepare.  (With the base shape alone, 1200 points in 40 columns took
+    // 0.76 ms in their own order, 0.71 sorted with one period per thread.)
+    auto weighs = [&](const FoldConfig& t) {
+        return mixed_ok && t.kind == KIND_BIN && t.block == base.block && t.rounds == 1;
+    };
+    int rc;
+    if ((rc = time_all(weighs)) != PF_OK) return rc;
+    float order_ms[2] = {1e30f, 1e30f};
+    for (const auto& c : timed)
+        order_ms[c.first.mixed] = std::min(order_ms[c.first.mixed], c.second);
+    const bool own_order = order_ms[1] < order_ms[0];
+    if ((rc = time_all([&](const FoldConfig& t) {
+             return !weighs(t) && !(mixed_ok && t.kind == KIND_BIN && t.mixed != own_order);
+         })) != PF_OK)
+        return rc;
     if (best.candidates == 0) return PF_OK;
     // Second pass over the candidates within 6% of the fastest: shapes that
     // close differ by less than the launch-to-launch spread of a ~1 ms
@@ -1142,7 +1164,6 @@ int tuned_config(pf_ctx* ctx, const Job& j, const FoldConfig& base, int cls, uin
     if (close.size() > 1)
         for (int round = 0; round < 3; round++)
             for (size_t i : close) {
-                int rc;
                 if ((rc = time_cand(timed[i].first, 1, timed[i].second)) != PF_OK) return rc;
             }
     for (const auto& c : timed) {

@@ -61,3 +61,30 @@ def test_large_histograms_may_share_them(monkeypatch, shared):
     alone._flags |= nat.PF_NO_TUNE
     np.testing.assert_array_equal(
         got, alone.periodograms(ts, ms, periods, np.zeros(1, np.float32)))
+
+
+@pytest.mark.parametrize("n_points, n_mag", [(50, 10), (120, 20), (200, 64)])
+def test_orders_are_weighed_before_the_shapes(monkeypatch, n_points, n_mag):
+    """The tuner times both point orders in the base shape's block and the other
+    shapes for the faster order alone: at most two samples more than the 12 of
+    one order, where both in every shape made 20."""
+    import re
+
+    from periodfind_b200 import _native as nat
+    from periodfind_b200 import gpu
+
+    ctx = nat.Context(0)
+    monkeypatch.setattr(nat, "default_context", lambda device=0: ctx)
+    rng = np.random.default_rng(3)
+    ts = [np.sort(rng.uniform(0, 900, n_points)).astype(np.float32) for _ in range(40)]
+    ms = [rng.uniform(0.01, 0.99, n_points).astype(np.float32) for _ in ts]
+    periods = np.geomspace(0.1, 30.0, 1000).astype(np.float32)
+    ce, alone = gpu.ConditionalEntropy(10, n_mag), gpu.ConditionalEntropy(10, n_mag)
+    got = ce.periodograms(ts, ms, periods, np.zeros(1, np.float32))
+    counts = [int(c) for c in re.findall(r"candidates=(\d+)", ctx.tuning_report())]
+    assert len(counts) == 1 and counts[0] <= 12 + 2, ctx.tuning_report()
+    other = nat.Context(0)
+    monkeypatch.setattr(nat, "default_context", lambda device=0: other)
+    alone._flags |= nat.PF_NO_TUNE
+    np.testing.assert_array_equal(
+        got, alone.periodograms(ts, ms, periods, np.zeros(1, np.float32)))
