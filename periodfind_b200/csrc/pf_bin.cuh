@@ -329,31 +329,42 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
 
     // The item covers ROUNDS x CELLS x BLOCK periods; in round r thread tid
     // takes periods p0 + (r * CELLS + c) * BLOCK + tid, c < CELLS, all at
-    // once.  Range guard for y = q * n * 2^20 over
-    // every round (uniform over the CTA).  The cell constants (1 / P as a
-    // double-double, pdt / 2P) are finite exactly when P is finite and non-zero
-    // and pdt is finite; non-finite periods or derivatives (device-pointer
-    // callers are not checked on the host) take the generic loop, whose bins
-    // are always clamped.
-    bool fin = isfinite(period_dt);
-    double my_pmin = INFINITY;
+    // once.  A dead cell repeats the last period.
+    auto period_at = [&](uint32_t j) -> uint32_t { return w.p0 + min(j, w.np - 1u); };
+    // Range guard for y = q * n * 2^20 over the `cells` periods of each thread
+    // of the warp from j on: |t_corr / P| is at most y (max|t| + |pdt| max|t|^2
+    // y / 2), y the largest |1/P| (infinite for a P of 0).  2: |q| < 2^19 as
+    // well, so the phase's 32 fraction bits come from one FMA; 1: the
+    // three-operation bin; 0: the exact sequence.  The cell constants (1 / P as a double-double, pdt / 2P) are
+    // finite exactly when P is finite and non-zero and pdt is finite;
+    // non-finite periods or derivatives (device-pointer callers are not
+    // checked on the host) take the exact sequence, whose bins are always
+    // clamped.
+    auto range_of = [&](uint32_t j, int cells) -> int {
+        uint32_t least = 0x7F800000u;  // the smallest |P|, 0 for what is not finite
 #pragma unroll
-    for (int r = 0; r < ROUNDS * CELLS; r++) {
-        const uint32_t j = (uint32_t)(r * BLOCK + tid);
-        const float per = p.periods[w.p0 + (j < w.np ? j : 0u)];
-        fin = fin && isfinite(per) && per != 0.0f;
-        my_pmin = fmin(my_pmin, fabs((double)per));
-    }
-    const double qb = cta_qbound_of<BLOCK>(p, my_pmin, period_dt);
+        for (int c = 0; c < cells; c++) {
+            const uint32_t per =
+                __float_as_uint(p.periods[period_at(j + (uint32_t)(c * BLOCK))]) & 0x7FFFFFFFu;
+            least = min(least, per < 0x7F800000u ? per : 0u);
+        }
+        const double y = __drcp_rn((double)__uint_as_float(__reduce_min_sync(0xffffffffu, least)));
+        const double tmax = (double)__uint_as_float(*p.tmax_bits);
+        const double q = y * __fma_rn(0.5 * fabs((double)period_dt) * tmax * tmax, y, tmax);
+        return q * (double)nP < 1073741824.0 ? q < 524288.0 ? 2 : 1 : 0;  // 2^30
+    };
+    // With one cell per thread the item's rounds share it; with several each
+    // round has its own, as the shortest of 512 periods would take all of them
+    // out of the fast range (2000 curves of 300 points x 1000 periods x 3
+    // derivatives, half the cells beyond it: AOV 1.74 -> 1.28 ms, CE 1.92 ->
+    // 1.73; AOV on the ragged plan within it 8.36 -> 8.24).
+    const int item_range = CELLS == 1 ? range_of((uint32_t)tid, ROUNDS) : 0;
     // The two FP64 divides of the AOV statistic that depend on the curve only.
     __shared__ double s_aov[2];
     if (ALGO == ALGO_AOV && !REF_STATS && tid == 0) {
         s_aov[0] = aov_xx_n(cd);
         s_aov[1] = aov_scale(n, nP);
     }
-    const bool fast = __syncthreads_and(fin ? 1 : 0) && qb * (double)nP < 1073741824.0;  // 2^30
-    // |q| < 2^19 as well: the phase's 32 fraction bits come from one FMA.
-    const bool fast32 = fast && qb < 524288.0;
 
     const double nd20 = (double)nP * 1048576.0;
     const uint32_t n_neg = 0u - nP;
@@ -426,18 +437,15 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
     for (int r = 0; r < ROUNDS; r++) {
     const uint32_t j0 = (uint32_t)(r * CELLS * BLOCK + tid);
     const bool active = j0 < w.np;  // a thread with any live cell runs all
-    auto cell_period = [&](int c) -> uint32_t {
-        const uint32_t j = j0 + (uint32_t)(c * BLOCK);
-        return w.p0 + (j < w.np ? j : 0u);
-    };
+    auto cell_period = [&](int c) -> uint32_t { return period_at(j0 + (uint32_t)(c * BLOCK)); };
+    const int range = CELLS == 1 ? item_range : range_of(j0, CELLS);
     // RN(1/P), times 2^32 where the one-FMA bin applies (exact), and pdt / 2P.
-    const double y_scale = fast32 ? 4294967296.0 : 1.0;
     double ys[CELLS], pc[CELLS];
 #pragma unroll
     for (int c = 0; c < CELLS; c++) {
         Cell s;
         cell_setup<FOLD_EXACT>(s, p.periods[cell_period(c)], period_dt);
-        ys[c] = s.yhi * y_scale;
+        ys[c] = s.yhi * (range == 2 ? 4294967296.0 : 1.0);
         pc[c] = s.c;
     }
     for (uint32_t k = 0; k < slots; k++)
@@ -635,7 +643,8 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
                             t = without_column(t);
                         }
                         uint32_t ev;
-                        const uint32_t row = bin_of(t, s.yhi * y_scale, s.c, ev);
+                        const uint32_t row =
+                            bin_of(t, s.yhi * (F32 ? 4294967296.0 : 1.0), s.c, ev);
                         const uint32_t ex =
                             exact_row(t, s, has_pdt_tag) - (F32 ? 0x80000000u : 0u);
                         if (ex != row) {
@@ -647,6 +656,18 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
                     }
                 }
             };
+            // Beyond the fast range: kSide cells side by side (three would take
+            // 8 registers more of the whole kernel), set up once per tile (the
+            // case above one after the other, set up for every run of points:
+            // CE 2.63 -> 1.92 ms).
+            constexpr int kSide = FAST || CELLS == 3 ? 1 : CELLS;
+            Cell slow[kSide];
+            auto set_up = [&](int c0) {
+#pragma unroll
+                for (int c = 0; c < kSide; c++)
+                    cell_setup<FOLD_EXACT>(slow[c], p.periods[cell_period(c0 + c)], period_dt);
+            };
+            if constexpr (!FAST && kSide == CELLS) set_up(0);
             // m points from tile position i (a multiple of 4).
             auto span = [&](uint32_t i, uint32_t m, uint32_t at, uint32_t inc) {
                 if constexpr (FAST) {
@@ -675,21 +696,23 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
                     }
                     if (k < m) group(G4{}, std::true_type{}, i + k, m - k, at, inc);
                 } else {
+                    constexpr int kUnroll = kSide == 1 ? 4 : 2;
 #pragma unroll 1
-                    for (int c = 0; c < CELLS; c++) {
-                        Cell s;
-                        cell_setup<FOLD_EXACT>(s, p.periods[cell_period(c)], period_dt);
-#pragma unroll 2
+                    for (int c0 = 0; c0 < CELLS; c0 += kSide) {
+                        if constexpr (kSide < CELLS) set_up(c0);
+#pragma unroll kUnroll
                         for (uint32_t k = 0; k < m; k++) {
                             double t = tile_t[i + k];
-                            uint32_t ak = at, ik = inc;
+                            uint32_t ak = at + c0 * BLOCK * 4, ik = inc;
                             if constexpr (MIXED) {
                                 ak = column_word(column_of(t));
                                 ik = column_unit(column_of(t));
                                 t = without_column(t);
                             }
-                            add(exact_row(t, s, has_pdt_tag), ak + c * BLOCK * 4, ik,
-                                ALGO == ALGO_AOV ? tile_a[i + k] : 0u);
+                            const uint32_t a = ALGO == ALGO_AOV ? tile_a[i + k] : 0u;
+#pragma unroll
+                            for (int c = 0; c < kSide; c++)
+                                add(exact_row(t, slow[c], has_pdt_tag), ak + c * BLOCK * 4, ik, a);
                         }
                     }
                 }
@@ -718,12 +741,12 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
         using T_ = std::true_type;
         using F_ = std::false_type;
         if (period_dt != 0.0f) {
-            if (fast32) body(T_{}, T_{}, T_{});
-            else if (fast) body(T_{}, T_{}, F_{});
+            if (range == 2) body(T_{}, T_{}, T_{});
+            else if (range == 1) body(T_{}, T_{}, F_{});
             else body(T_{}, F_{}, F_{});
         } else {
-            if (fast32) body(F_{}, T_{}, T_{});
-            else if (fast) body(F_{}, T_{}, F_{});
+            if (range == 2) body(F_{}, T_{}, T_{});
+            else if (range == 1) body(F_{}, T_{}, F_{});
             else body(F_{}, F_{}, F_{});
         }
     }
