@@ -573,6 +573,9 @@ int validate_common(pf_ctx* ctx, const Job& j) {
         return fail(ctx, PF_EINVAL, "peak outputs are NULL");
     if (j.stats && (!j.out_stats || (j.n_top > 0 && (!j.out_idx || !j.out_val))))
         return fail(ctx, PF_EINVAL, "stats outputs are NULL");
+    // The accepted row lengths (17066 summation leaves, about 2.1 million
+    // cells) are those of an earlier layout of 12 bytes a leaf, kept so that no
+    // call changes; the kernel's 4 << tree_depth bytes are 128 KB at most there.
     if (j.stats && j.n_per * j.n_pdt > 0 && stats_leaf_count((uint32_t)std::min<uint64_t>(
                                                    j.n_per * j.n_pdt, 0xFFFFFFFFull)) *
                                                    12ull > 200ull * 1024ull)
@@ -677,8 +680,8 @@ FoldConfig choose_config(pf_ctx* ctx, const Job& j, uint32_t max_len, bool& ok) 
 // reference's quotient folded / bin_size differs from frac(q') * n by less
 // than 2 ulp (f32 divide) + n * 2^-23 (bin width rounding) + n * 2^-25
 // (f64 -> f32 rounding of the phase) + 2^-20 (q' = t * RN(1/P) against
-// RN(t / P): 2 ulp(q) * n <= 2^-20 while |q| * n < 2^30), plus two units of
-// margin.
+// RN(t / P): 2 ulp(q) * n <= 2^-20 while |q| * n < 2^30), plus two units, of
+// which AOV's one-FMA derivative correction takes up to an eighth (2^-23).
 uint32_t edge_guard(uint32_t n) {
     int cl = 0;
     while ((1u << cl) < n + 1u) cl++;
@@ -868,10 +871,11 @@ uint64_t queue_items(const Job& j, uint64_t n_curves, int per_item) {
 // The non-uniform FFT is a candidate from this many frequencies on (a block
 // costs the same however few of its kNufftModes are asked for).
 constexpr uint64_t kNufftMinFreqs = 1024;
-// And for the classes of at least 64 points, where its rounding is no larger
-// than the direct sums': power error against FP64 (2-norm) 2.9e-7 against 3.2e-7
-// at 64 points, 2.6e-7 against 5.0e-7 at 256, 4.0e-7 against 7.9e-6 at 16384; at
-// 20 and 33 points 3.2e-7 against 2.8e-7 and 3.1e-7.
+// And for the classes of at least 64 points, where its rounding is clearly below
+// the direct sums': power error against FP64 (2-norm) 2.7e-7 against 3.3e-7 at 64
+// points, 2.6e-7 against 4.9e-7 at 256, 1.8e-7 against 3.5e-6 at 16384.  At 20
+// points (2.8e-7 against 2.9e-7) the two are level, and curves of a few points,
+// near-singular at many frequencies, keep the direct form's values.
 constexpr int kNufftClassMin = 1;
 
 // Frequencies of a grid, as far as the tuner's choice depends on them: the
@@ -2534,6 +2538,7 @@ int pf_prepare_mags_dev(pf_ctx* ctx, const float* d_mags, const int64_t* offsets
         if (kind == PF_PREP_CENTER && len > 0)
             leaf_cap = std::max(leaf_cap, stats_leaf_count((uint32_t)len));
     }
+    // (the accepted lengths as for the device statistics)
     if ((size_t)leaf_cap * 12 > 200u * 1024u)
         return fail(ctx, PF_EUNSUPPORTED, "a curve is too long for the device mean");
     if (offsets[n_curves] > offsets[0] && (!d_mags || !d_out))

@@ -205,12 +205,12 @@ __global__ void __launch_bounds__(BLOCK)
 // (30 curves x 2000 points x 2000 periods from 0.0005 on: 138 us; a branch and
 // the exact sequence at every point took 333, with one period per thread 223).
 //
-// Bound: the shared-memory pipe, 96% busy for FPW (per evaluation half a
-// 128-bit broadcast load, an 8-byte load and an 8-byte store), 75% for BLS.
+// Bound: the shared-memory pipe, 97% busy for FPW (per evaluation half a
+// 128-bit broadcast load, an 8-byte load and an 8-byte store), 76% for BLS.
 // FPW(10) with uncertainties, 100 curves x 4096 points x 10000 periods x 2:
-// 4.81 ms, the call from host arrays 9.35 -> 6.70 ms; BLS(50), 150 x 1500 x
-// 10000, whose 1250 windows per cell cost as much as its points: the call 5.50
-// -> 3.86 ms (4.15 ms with one window loop and a select per wrap).
+// 4.77 ms, the call from host arrays 9.02 -> 6.62 ms; BLS(50), 150 x 1500 x
+// 10000, whose 1250 windows per cell cost as much as its points: the call 5.46
+// -> 3.74 ms (4.15 ms with one window loop and a select per wrap).
 template <int BLOCK, bool BLS, int CELLS>
 __global__ void __launch_bounds__(BLOCK)
     fpw_chosen_kernel(const FpwParams p, uint32_t tiles_per_row) {

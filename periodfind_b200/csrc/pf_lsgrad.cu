@@ -435,7 +435,7 @@ __device__ __forceinline__ float phase_fast(F2 f, float dh, float dl) {
 // point tile 0 also write the frequency gradient g_k * dP/domega_k.  One
 // 128-bit broadcast load (frequency pair, weights) serves the thread's
 // points; the sum over a staged tile is added to the total (two levels).
-// Bound: the MUFU unit (86% of its rate with one point per thread; 100 curves x
+// Bound: the MUFU unit (85% of its rate with one point per thread; 100 curves x
 // 2048 points x 20000 frequencies in 2.26 ms), with a few points the latency of
 // a frequency: 16 of them at once and two chains of sums (one curve of 100
 // points x 20000: 453 -> 389 us, 420 with four scalar loads per frequency).
