@@ -353,12 +353,13 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
         const double q = y * __fma_rn(0.5 * fabs((double)period_dt) * tmax * tmax, y, tmax);
         return q * (double)nP < 1073741824.0 ? q < 524288.0 ? 2 : 1 : 0;  // 2^30
     };
-    // With one cell per thread the item's rounds share it; with several each
-    // round has its own, as the shortest of 512 periods would take all of them
+    // With one cell per thread the item's rounds share it; with several each of
+    // its rounds has its own, as the shortest of 512 periods would take all of them
     // out of the fast range (2000 curves of 300 points x 1000 periods x 3
     // derivatives, half the cells beyond it: AOV 1.74 -> 1.28 ms, CE 1.92 ->
     // 1.73; AOV on the ragged plan within it 8.36 -> 8.24).
-    const int item_range = CELLS == 1 ? range_of((uint32_t)tid, ROUNDS) : 0;
+    constexpr bool kItemRange = CELLS == 1 || ROUNDS == 1;
+    const int item_range = kItemRange ? range_of((uint32_t)tid, ROUNDS * CELLS) : 0;
     // The two FP64 divides of the AOV statistic that depend on the curve only.
     __shared__ double s_aov[2];
     if (ALGO == ALGO_AOV && !REF_STATS && tid == 0) {
@@ -438,7 +439,7 @@ __device__ __forceinline__ void bin_item(const FoldParams& p, const WorkItem w, 
     const uint32_t j0 = (uint32_t)(r * CELLS * BLOCK + tid);
     const bool active = j0 < w.np;  // a thread with any live cell runs all
     auto cell_period = [&](int c) -> uint32_t { return period_at(j0 + (uint32_t)(c * BLOCK)); };
-    const int range = CELLS == 1 ? item_range : range_of(j0, CELLS);
+    const int range = kItemRange ? item_range : range_of(j0, CELLS);
     // RN(1/P), times 2^32 where the one-FMA bin applies (exact), and pdt / 2P.
     double ys[CELLS], pc[CELLS];
 #pragma unroll
